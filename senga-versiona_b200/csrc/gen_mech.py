@@ -262,7 +262,51 @@ def poly_expr(coefs, var):
 
 
 def sel(it_var, a, b):
-    return a if a == b else f"({it_var} ? {b} : {a})"
+    """The value of interval it_var: a select, or the literal itself inside a
+    function whose template mode IM fixes the interval (see `modes`)."""
+    return a if a == b else f"(IM == 0 ? {a} : IM == 1 ? {b} : {it_var} ? {b} : {a})"
+
+
+# Reverse rates as products of exp(Gibbs function) factors need every partial
+# product in range over these temperatures (the tables start at 300 K).
+GIB_T, GIB_LIMIT = (100.0, 200.0, 300.0, 1000.0, 3000.0, 6000.0), 650.0
+
+
+def gibbs(c, s, it, T):
+    g = c["amolgb"][s][it]
+    np_, nh, nsy = c["ncpoly"][s][it], c["ncenth"][s][it], c["ncenpy"][s][it]
+    v = g[np_ - 1]
+    for q in range(np_ - 1, 0, -1):
+        v = g[q - 1] + v * T
+    return g[nh - 1] / T - g[nsy - 1] * math.log(T) - v
+
+
+def gibbs_products_in_range(c):
+    """True when every reverse rate can be formed from exp(g_k) factors: the
+    exponents of all factors and partial products, in the order in which they
+    are multiplied, stay below GIB_LIMIT in size (of 709)."""
+    for st in range(c["nstep"]):
+        if not c["mglist"][st]:
+            continue
+        for T in GIB_T:
+            total = 0.0
+            for q, (sp, _) in enumerate(c["nsspec"][st]):
+                d, s = c["diffmu"][st][q], sp - 1
+                it = 1 if c["ntint"][s] > 1 and T > c["tinthi"][s][0] else 0
+                total += d * gibbs(c, s, it, T)
+                if d != int(d) or max(abs(gibbs(c, s, it, T)), abs(total)) > GIB_LIMIT:
+                    return False
+    return True
+
+
+def groups_of(rows):
+    """Rows of polynomial coefficients grouped by equal coefficients past the
+    constant one: [(representative, [members])]. exp of a group's polynomials
+    is one exp times exp(difference of the constants)."""
+    seen = {}
+    for k, r in rows:
+        seen.setdefault(tuple(r[1:]), []).append(k)
+    return [(m[0], m) for m in seen.values()]
 
 
 def gen(tag, c, d):
@@ -276,9 +320,17 @@ def gen(tag, c, d):
     w("  __device__ __forceinline__ bool has(int) const { return true; }")
     w("  __device__ __forceinline__ int count() const { return NS; }")
     # ---- temper coefficients
-    w("  __device__ __forceinline__ void temper_coeffs(const double (&ry)[NS], uint64_t itn0, double (&tc)[6], double (&td)[6], double& rmix) const {")
+    # Functions with interval-dependent literals come in three modes IM: every
+    # species in interval 0, every one in interval 1, or mixed (a select per
+    # literal). Points away from the breakpoint take the first two, where no
+    # select and no second literal is left.
+    allhi = sum(1 << (2 * s) for s in range(ns) if c["ntint"][s] > 1)
+    w(f"  static constexpr uint64_t kAllHigh = {allhi}ull;")
+    w("  static __device__ __forceinline__ int mode(uint64_t itn) { return itn == 0 ? 0 : itn == kAllHigh ? 1 : 2; }")
+    w("  template <int IM>")
+    w("  __device__ __forceinline__ void temper_coeffs_m(const double (&ry)[NS], uint64_t itn0, double (&tc)[6], double (&td)[6], double& rmix) const {")
     for s in range(ns):
-        w(f"    {{ const int it = (itn0 >> {2 * s}) & 1; const double y = ry[{s}];")
+        w(f"    {{ const int it = (itn0 >> {2 * s}) & 1; (void)it; const double y = ry[{s}];")
         nint = c["ntint"][s]
         def cv(table, q):
             a = table[s][0][q]
@@ -296,15 +348,29 @@ def gen(tag, c, d):
             w(f"      td[{icp}] = td[{icp}] + y * {cv(c['amascp'], icp - 1)};")
         w(f"      rmix = rmix + y * {h(c['rgspec'][s])}; }}")
     w("  }")
+    w("  __device__ __forceinline__ void temper_coeffs(const double (&ry)[NS], uint64_t itn0, double (&tc)[6], double (&td)[6], double& rmix) const {")
+    w("    const int im = mode(itn0);")
+    w("    if (im == 0) temper_coeffs_m<0>(ry, itn0, tc, td, rmix);")
+    w("    else if (im == 1) temper_coeffs_m<1>(ry, itn0, tc, td, rmix);")
+    w("    else temper_coeffs_m<2>(ry, itn0, tc, td, rmix);")
+    w("  }")
     # ---- locate + cp
     w("  __device__ __forceinline__ void locate(double T, const double (&ry)[NS], uint64_t& itn, double& cpsum) const {")
-    w("    itn = 0; cpsum = 0.0;")
+    w("    itn = 0;")
+    for s in range(ns):
+        if c["ntint"][s] > 1:
+            w(f"    itn += (uint64_t)(T > {h(c['tinthi'][s][0])} ? 1 : 0) << {2 * s};")
+    w("    const int im = mode(itn);")
+    w("    if (im == 0) cp_m<0>(T, ry, itn, cpsum);")
+    w("    else if (im == 1) cp_m<1>(T, ry, itn, cpsum);")
+    w("    else cp_m<2>(T, ry, itn, cpsum);")
+    w("  }")
+    w("  template <int IM>")
+    w("  __device__ __forceinline__ void cp_m(double T, const double (&ry)[NS], uint64_t itn, double& cpsum) const {")
+    w("    cpsum = 0.0;")
     for s in range(ns):
         np_ = c["ncpoly"][s][0]
-        if c["ntint"][s] > 1:
-            w(f"    {{ const int it = T > {h(c['tinthi'][s][0])} ? 1 : 0; itn += (uint64_t)it << {2 * s};")
-        else:
-            w("    { const int it = 0; (void)it;")
+        w(f"    {{ const int it = (itn >> {2 * s}) & 1; (void)it;")
         cp0, cp1 = c["amascp"][s][0], (c["amascp"][s][1] if c["ntint"][s] > 1 else c["amascp"][s][0])
         w(f"      double v = {sel('it', h(cp0[np_ - 1]), h(cp1[np_ - 1]))};")
         for icp in range(np_ - 1, 0, -1):
@@ -322,44 +388,83 @@ def gen(tag, c, d):
     w("  __device__ __forceinline__ void mixture(double T, double p, double rho, const double (&ry)[NS], const double (&y)[NS], double& lam, double (&rd)[NS], double& mu) const {")
     if mavt:
         w(f"    const double lt = log(T / {h(d['tdifgb'])});")
-        w("    double c1 = 0.0, c2 = 0.0, c3 = 0.0;")
+        w("    double c1 = 0.0, c3 = 0.0;")
+        # conductivity: sum fm lk and sum fm / lk; the second as one running
+        # fraction num / den (all terms positive), one division in place of
+        # nine; lambda = (sum fm lk / sum fm + sum fm / (sum fm / lk)) / 2
+        w("    double num = 0.0, den = 1.0;")
         for s in range(ns):
             w(f"    {{ const double lk = exp({poly_expr(d['condco'][s], 'lt')}); const double fm = ry[{s}] * {h(c['ovwmol'][s])};")
-            w("      c1 = c1 + fm * lk; c2 = c2 + fm / lk; c3 = c3 + fm; }")
-        w("    c3 = 1.0 / c3; c1 = c1 * c3; c2 = c2 * c3;")
-        w("    lam = 0.5 * (c1 + 1.0 / c2);")
-        w("    const double wmix = rho * c3;")
-        w(f"    const double povr = p / {h(d['pdifgb'])};")
+            w("      c1 = c1 + fm * lk; num = num * lk + fm * den; den = den * lk; c3 = c3 + fm; }")
+        w("    lam = 0.5 * (c1 / c3 + c3 * (den / num));")
+        for s in range(ns):
+            w(f"    const double x{s} = y[{s}] * {h(c['ovwmol'][s])};")
         # Wilke viscosity before the mixture diffusivities, so that the nine
-        # rho D_k are formed last and stored right after: the square roots
-        # and the diffusivity sums are never live together (fewer registers);
-        # mu_k is taken as sqrt(mu_k)^2 (within an ulp of mu_k)
+        # rho D_k are formed last and stored right after (fewer registers).
+        # sqrt(mu_k) = exp(poly / 2), one exp per group of species whose
+        # polynomials differ in the constant only; the combination sum
+        # sum_t x_t w1 (1 + sq_s rq_t w2)^2 expanded in powers of sq_s (three
+        # fused operations per pair, all terms positive); the nine quotients
+        # as one running fraction.
+        for b, mem in groups_of([(s, d["viscco"][s]) for s in range(ns)]):
+            half = [0.5 * v for v in d["viscco"][b]]
+            w(f"    const double sq{b} = exp({poly_expr(half, 'lt')}); const double rq{b} = 1.0 / sq{b};")
+            for t in mem[1:]:
+                r = 0.5 * (d["viscco"][t][0] - d["viscco"][b][0])
+                w(f"    const double sq{t} = sq{b} * {h(math.exp(r))}; const double rq{t} = rq{b} * {h(math.exp(-r))};")
+        for t in range(ns):
+            w(f"    const double xr{t} = x{t} * rq{t}; const double xq{t} = xr{t} * rq{t};")
+        w("    num = 0.0; den = 1.0;")
         for s in range(ns):
-            w(f"    const double sq{s} = sqrt(exp({poly_expr(d['viscco'][s], 'lt')})); const double rq{s} = 1.0 / sq{s};")
-        w("    mu = 0.0;")
-        for s in range(ns):
-            w("    { double cc = 0.0, fw;")
+            w("    { double ca = 0.0, cb = 0.0, cc = 0.0;")
             for t in range(ns):
-                w(f"      fw = 1.0 + sq{s} * rq{t} * {h(d['wilko2'][s][t])}; fw = {h(d['wilko1'][s][t])} * fw * fw; cc = cc + y[{t}] * {h(c['ovwmol'][t])} * fw;")
-            w(f"      mu = mu + y[{s}] * {h(c['ovwmol'][s])} * ((sq{s} * sq{s}) / cc); }}")
+                w1, w2 = d["wilko1"][s][t], d["wilko2"][s][t]
+                w(f"      ca += x{t} * {h(w1)}; cb += xr{t} * {h(2.0 * w1 * w2)}; cc += xq{t} * {h(w1 * w2 * w2)};")
+            w(f"      ca = ca + sq{s} * (cb + sq{s} * cc);")
+            w(f"      num = num * ca + x{s} * (sq{s} * sq{s}) * den; den = den * ca; }}")
+        w("    mu = num / den;")
+        # mixture diffusivities: rho D_s = rho (sumy - y_s) / (den_s W_mix p/p0),
+        # den_s = sum_t x_t exp(-poly_st); one exp per group of pairs whose
+        # polynomials differ in the constant only, and the quotients three at
+        # a time from one division
         w("    double sumy = 0.0;")
         for s in range(ns):
-            w(f"    sumy += y[{s}] + {h(DFCTOL)};")
+            w(f"    const double ye{s} = y[{s}] + {h(DFCTOL)}; sumy += ye{s};")
         for s in range(ns):
+            w(f"    const double xe{s} = ye{s} * {h(c['ovwmol'][s])};")
             w(f"    double den{s} = 0.0;")
-        for s in range(ns):
-            for t in range(s + 1, ns):
-                w(f"    {{ const double inv = exp(-{poly_expr(d['diffco'][s][t], 'lt')}) * povr;")
-                w(f"      den{s} += (y[{t}] + {h(DFCTOL)}) * {h(c['ovwmol'][t])} * inv;")
-                w(f"      den{t} += (y[{s}] + {h(DFCTOL)}) * {h(c['ovwmol'][s])} * inv; }}")
-        for s in range(ns):
-            w(f"    rd[{s}] = rho * (sumy - (y[{s}] + {h(DFCTOL)})) / (den{s} * wmix);")
+        pairs = [((s, t), d["diffco"][s][t]) for s in range(ns) for t in range(s + 1, ns)]
+        for (bs, bt), mem in groups_of(pairs):
+            w(f"    {{ const double gx = exp(-{poly_expr(d['diffco'][bs][bt], 'lt')});")
+            for s, t in mem:
+                r = d["diffco"][s][t][0] - d["diffco"][bs][bt][0]
+                f = "gx" if r == 0.0 else f"(gx * {h(math.exp(-r))})"
+                w(f"      {{ const double inv = {f}; den{s} += xe{t} * inv; den{t} += xe{s} * inv; }}")
+            w("    }")
+        w(f"    const double kd = c3 * {h(d['pdifgb'])} / p;")
+        for s0 in range(0, ns, 3):
+            k = list(range(s0, min(s0 + 3, ns)))
+            if len(k) == 3:
+                a_, b_, e_ = k
+                w(f"    {{ const double ab = den{a_} * den{b_}; const double iv = kd / (ab * den{e_}); const double ie = iv * den{e_};")
+                w(f"      rd[{a_}] = (sumy - ye{a_}) * (ie * den{b_}); rd[{b_}] = (sumy - ye{b_}) * (ie * den{a_}); rd[{e_}] = (sumy - ye{e_}) * (iv * ab); }}")
+            else:
+                for s in k:
+                    w(f"    rd[{s}] = (sumy - ye{s}) * (kd / den{s});")
+        w("    (void)rho;")
     else:
         w("    (void)T; (void)p; (void)rho; (void)ry; (void)y; lam = 0.0; mu = 0.0;")
         w("    for (int s = 0; s < NS; ++s) rd[s] = 0.0;")
     w("  }")
     # ---- enthalpy
     w("  __device__ __forceinline__ void enthalpy(double T, uint64_t itn, double (&hk)[NS]) const {")
+    w("    const int im = mode(itn);")
+    w("    if (im == 0) enthalpy_m<0>(T, itn, hk);")
+    w("    else if (im == 1) enthalpy_m<1>(T, itn, hk);")
+    w("    else enthalpy_m<2>(T, itn, hk);")
+    w("  }")
+    w("  template <int IM>")
+    w("  __device__ __forceinline__ void enthalpy_m(double T, uint64_t itn, double (&hk)[NS]) const {")
     for s in range(ns):
         np_, nh = c["ncpoly"][s][0], c["ncenth"][s][0]
         a0 = c["amasch"][s][0]
@@ -370,56 +475,108 @@ def gen(tag, c, d):
         w(f"      hk[{s}] = {sel('it', h(a0[nh - 1]), h(a1[nh - 1]))} + v * T; }}")
     w("  }")
     # ---- CHRATE
-    w("  __device__ __forceinline__ void chrate(double T, uint64_t itn, const double (&ry)[NS], double (&rate)[NS]) const {")
-    w("    const double lnT = log(T); const double ovT = 1.0 / T; (void)itn;")
-    for s in range(ns):
-        w(f"    rate[{s}] = 0.0;")
     need_gibbs = c["ngibb"] > 0
+    products = need_gibbs and gibbs_products_in_range(c)
+    used = sorted({sp - 1 for st in range(c["nstep"]) if c["mglist"][st] for sp, _ in c["nsspec"][st]})
     if need_gibbs:
-        for s in range(ns):
+        # g_k of every species that a reversible step changes
+        w("  template <int IM>")
+        w("  __device__ __forceinline__ void gibbs_m(double T, double ovT, double lnT, uint64_t itn, double (&g)[NS]) const {")
+        for s in used:
             np_, nh, nsy = c["ncpoly"][s][0], c["ncenth"][s][0], c["ncenpy"][s][0]
             g0 = c["amolgb"][s][0]
             g1 = c["amolgb"][s][1] if c["ntint"][s] > 1 else g0
-            w(f"    double gib{s}; {{ const int it = (itn >> {2 * s}) & 1; (void)it; double v = {sel('it', h(g0[np_ - 1]), h(g1[np_ - 1]))};")
+            w(f"    {{ const int it = (itn >> {2 * s}) & 1; (void)it; double v = {sel('it', h(g0[np_ - 1]), h(g1[np_ - 1]))};")
             for icp in range(np_ - 1, 0, -1):
                 w(f"      v = {sel('it', h(g0[icp - 1]), h(g1[icp - 1]))} + v * T;")
-            w(f"      gib{s} = {sel('it', h(g0[nh - 1]), h(g1[nh - 1]))} / T - {sel('it', h(g0[nsy - 1]), h(g1[nsy - 1]))} * lnT - v; }}")
+            w(f"      g[{s}] = {sel('it', h(g0[nh - 1]), h(g1[nh - 1]))} * ovT - {sel('it', h(g0[nsy - 1]), h(g1[nsy - 1]))} * lnT - v; }}")
+        w("  }")
+    w("  __device__ __forceinline__ void chrate(double T, uint64_t itn, const double (&ry)[NS], double (&rate)[NS]) const {")
+    w("    const double lnT = log(T); const double ovT = 1.0 / T; (void)itn; (void)lnT;")
+    for s in range(ns):
+        w(f"    rate[{s}] = 0.0;")
+    if need_gibbs:
+        w("    double gib[NS];")
+        w("    const int im = mode(itn);")
+        w("    if (im == 0) gibbs_m<0>(T, ovT, lnT, itn, gib);")
+        w("    else if (im == 1) gibbs_m<1>(T, ovT, lnT, itn, gib);")
+        w("    else gibbs_m<2>(T, ovT, lnT, itn, gib);")
+    if products:
+        # exp(sum dmu_k g_k) of a reverse rate as a product of exp(g_k) and
+        # their reciprocals: one exp per species instead of one per step (the
+        # exponents are small enough that every product stays in range)
+        for s in used:
+            w(f"    const double ep{s} = exp(gib[{s}]);")
+        neg = {sp - 1 for st in range(c["nstep"]) if c["mglist"][st] for q, (sp, _) in enumerate(c["nsspec"][st]) if c["diffmu"][st][q] < 0}
+        for s in sorted(neg):
+            w(f"    const double en{s} = 1.0 / ep{s};")
+    for s in sorted({sp - 1 for st in range(c["nstep"]) for key in ("nrspec", "npspec") for sp, _ in c[key][st]}):
+        w(f"    const double cm{s} = fmax(ry[{s}] * {h(c['ovwmol'][s])}, 0.0);")
+    # rate constants exp(A + n ln T - E / T): a literal where n = E = 0, powers
+    # of T for an integer n with E = 0, one exp(-E / T) shared by the steps of
+    # equal E and integer n, else its own exp
+    def power(n):
+        n = int(n)
+        return " * ".join(["T"] * n if n > 0 else ["ovT"] * -n)
+
+    small = lambda n: n == int(n) and abs(n) <= 3  # noqa: E731
+    esteps = {}
+    for st in range(c["nstep"]):
+        A, nexp, E = c["rparam"][st]
+        if E != 0.0 and small(nexp):
+            esteps.setdefault(E, []).append(st)
+    shared = {E: k for k, (E, sts) in enumerate(esteps.items()) if len(sts) > 1}
+    for E, k in shared.items():
+        w(f"    const double ee{k} = exp(-{h(E)} * ovT);")
     w("    double s3 = 0.0; (void)s3;")
     for st in range(c["nstep"]):
         w(f"    {{ // step {st + 1}")
         ib = c["mblist"][st]
         flthrd = True
         if ib != 0:
-            terms = " + ".join(f"ry[{s}] * {h(c['ovwmol'][s] * c['effy3b'][ib - 1][s])}" for s in range(ns))
             w("      s3 = 0.0;")
             for s in range(ns):
                 w(f"      s3 += ry[{s}] * {h(c['ovwmol'][s] * c['effy3b'][ib - 1][s])};")
         A, nexp, E = c["rparam"][st]
-        w(f"      double s2 = {h(A)} + {h(nexp)} * lnT - {h(E)} * ovT;")
-        w("      double s1 = exp(s2);")
+        if E == 0.0 and small(nexp):
+            f = [h(math.exp(A))] + ([power(nexp)] if nexp else [])
+            w(f"      double s1 = {' * '.join(f)};")
+        elif E in shared and small(nexp):
+            f = [h(math.exp(A)), f"ee{shared[E]}"] + ([power(nexp)] if nexp else [])
+            w(f"      double s1 = {' * '.join(f)};")
+        else:
+            f = h(A) + (f" + {h(nexp)} * lnT" if nexp else "") + (f" - {h(E)} * ovT" if E else "")
+            w(f"      double s1 = exp({f});")
         if c["mllist"][st] != 0:
             L = c["rclind"][c["mllist"][st] - 1]
             import struct
             flc = struct.unpack("f", struct.pack("f", L[3]))[0]  # REAL (single) in the reference
             w(f"      {{ const double s4 = exp({h(L[0])} + {h(L[1])} * lnT - {h(L[2])} * ovT);")
             w("        const double pr = s3 * s4 / s1;")
-            w(f"        s1 = s1 * ({h(flc)} * pr / (1.0 + pr)); s2 = log(s1); }}")
+            w(f"        s1 = s1 * ({h(flc)} * pr / (1.0 + pr)); }}")
             flthrd = False
+        if c["mglist"][st] != 0:
+            if products:
+                w("      double s2 = s1;")
+                for q, (sp, _) in enumerate(c["nsspec"][st]):
+                    dmu = int(c["diffmu"][st][q])
+                    for _ in range(abs(dmu)):
+                        w(f"      s2 = s2 * {'ep' if dmu > 0 else 'en'}{sp - 1};")
+            else:
+                w("      double s2 = log(s1);")
+                for q, (sp, _) in enumerate(c["nsspec"][st]):
+                    w(f"      s2 = s2 + {h(c['diffmu'][st][q])} * gib[{sp - 1}];")
+                w("      s2 = exp(s2);")
         for sp, _ in c["nrspec"][st]:
-            w(f"      s1 = s1 * fmax(ry[{sp - 1}] * {h(c['ovwmol'][sp - 1])}, 0.0);")
+            w(f"      s1 = s1 * cm{sp - 1};")
         for sp, cf in c["nrcpec"][st]:
             w(f"      {{ double fn = fmax(ry[{sp - 1}] * {h(c['ovwmol'][sp - 1])}, 1.0e-30); fn = exp({h(cf)} * log(fn)); s1 = s1 * (fn / (1.0 + 1.0e-15 * fn)); }}")
         if c["mglist"][st] != 0:
-            for q, (sp, _) in enumerate(c["nsspec"][st]):
-                w(f"      s2 = s2 + {h(c['diffmu'][st][q])} * gib{sp - 1};")
-            w("      s2 = exp(s2);")
             for sp, _ in c["npspec"][st]:
-                w(f"      s2 = s2 * fmax(ry[{sp - 1}] * {h(c['ovwmol'][sp - 1])}, 0.0);")
+                w(f"      s2 = s2 * cm{sp - 1};")
             for sp, cf in c["npcpec"][st]:
                 w(f"      {{ double fn = fmax(ry[{sp - 1}] * {h(c['ovwmol'][sp - 1])}, 1.0e-30); fn = exp({h(cf)} * log(fn)); s2 = s2 * (fn / (1.0 + 1.0e-15 * fn)); }}")
             w("      s1 = s1 - s2;")
-        else:
-            w("      (void)s2;")
         if ib != 0 and flthrd:
             w("      s1 = s1 * s3;")
         for q, (sp, _) in enumerate(c["nsspec"][st]):

@@ -42,10 +42,13 @@ __global__ void __launch_bounds__(kBlock, ThermoOcc<M>::blocks) k_thermo(Geo g, 
   if (q >= g.n) return;
   thermo_point(g, f, m, q);
 }
-// The two halves of the thermochemistry: PART 1 at three blocks per SM (the
-// mixture-averaged transport wants ~128 registers; at 80 it spills some, and
-// the extra warps still win: 5.17 against 5.35 ms per substage on the 256^3
-// H2 box), PART 2 (CHRATE) at three.
+// The two halves of the thermochemistry, each at three blocks per SM. Both
+// are bound by the FP64 pipe (about 2600 and 1300 FP64 instructions a point
+// when every step, pair and quotient had its own exp and divide); the
+// generated forms share one exp among polynomials that differ in a constant,
+// form reverse rates from one exp per species, and sum quotients as running
+// fractions (gen_mech.py). 256^3 H2 box: part 1 3.76 -> 2.52, part 2 1.69 ->
+// 1.17 ms per launch; 32^3: 17.3 -> 10.4 and 7.6 -> 6.2 us.
 #ifndef SENGA_THERMO_P1_MINB
 #define SENGA_THERMO_P1_MINB 3
 #endif

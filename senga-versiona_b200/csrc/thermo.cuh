@@ -319,7 +319,8 @@ __device__ __forceinline__ void thermo_point(const Geo& g, const Fields& f, cons
   const double rho = U[q], ru = U[n + q], rv = U[2 * n + q], rw = U[3 * n + q], re = U[4 * n + q];
 
   // ---- TEMPER: Newton inversion of e(T) from the previous T ----
-  const double ukuk = (ru * ru + rv * rv + rw * rw) / rho;
+  const double orho = 1.0 / rho;  // one reciprocal for the 13 quotients by rho
+  const double ukuk = (ru * ru + rv * rv + rw * rw) * orho;
   double tc[6], td[6];
   tc[0] = 0.5 * ukuk - re;
 #pragma unroll
@@ -351,7 +352,7 @@ __device__ __forceinline__ void thermo_point(const Geo& g, const Fields& f, cons
   uint64_t itn;
   double cpm;
   m.locate(T, ry, itn, cpm);
-  cpm = cpm / rho;
+  cpm = cpm * orho;
   const double p = T * rmix;
   f.t[q] = T;
   itn_store(f.itn, n, q, m.count(), itn);
@@ -365,18 +366,18 @@ __device__ __forceinline__ void thermo_point(const Geo& g, const Fields& f, cons
   double y[NS];
 #pragma unroll
   for (int s = 0; s < NS; ++s) {
-    y[s] = ry[s] / rho;
+    y[s] = ry[s] * orho;
     if (m.has(s)) f.y[s * n + q] = y[s];
   }
-  f.vel[q] = ru / rho;
-  f.vel[n + q] = rv / rho;
-  f.vel[2 * n + q] = rw / rho;
+  f.vel[q] = ru * orho;
+  f.vel[n + q] = rv * orho;
+  f.vel[2 * n + q] = rw * orho;
   if (f.mom) {
     f.mom[q] = ru;
     f.mom[n + q] = rv;
     f.mom[2 * n + q] = rw;
   }
-  f.e[q] = re / rho;
+  f.e[q] = re * orho;
 
   // ---- transport properties ----
   if (!M::MAVT) {
