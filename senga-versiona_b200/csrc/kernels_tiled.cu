@@ -31,31 +31,54 @@ using namespace tile;
 // ---- single-box launches: one CTA per tile ----
 // B: plain fields staged by bulk copies on the TMA engine (all-periodic
 // boxes of even nx, one context, 16-byte aligned fields; the launcher checks)
-template <bool P, bool B>
-__global__ void __launch_bounds__(FX* FY, SENGA_FLOW_MINB) k_flow_t(Geo g, Fields f, ZDec zd) {
-  extern __shared__ __align__(16) double sm[];
-  __shared__ Folds<FX, FY, FZ> fo;
+template <bool P, bool B, class TS = Tile3>
+__global__ void __launch_bounds__(TS::X* TS::Y, SENGA_FLOW_MINB * 256 / (TS::X * TS::Y))
+    k_flow_t(Geo g, Fields f, ZDec zd) {
+  extern __shared__ __align__(128) double sm[];
+  __shared__ Folds<TS::X, TS::Y, TS::Z> fo;
   __shared__ uint64_t bar;
-  flow_tile<P, B>(g, f, Origin{(int)blockIdx.x * FX, (int)blockIdx.y * FY, (int)blockIdx.z * FZ}, sm, fo, zd, &bar);
+  flow_tile<P, B, true, TS>(g, f, Origin{(int)blockIdx.x * TS::X, (int)blockIdx.y * TS::Y, (int)blockIdx.z * TS::Z},
+                            sm, fo, zd, &bar);
 }
-template <bool P, int M>
-__global__ void __launch_bounds__(SX_* SY_, SENGA_SPEC_MINB)
+template <bool P, int M, class TS = Tile3>
+__global__ void __launch_bounds__(TS::X* TS::Y, SENGA_SPEC_MINB * 256 / (TS::X * TS::Y))
     k_species_t(Geo g, Fields f, int nspec, ZDec zd, const __grid_constant__ SpecMaps tm) {
   extern __shared__ __align__(128) double sm[];
-  __shared__ Folds<SX_, SY_, SZ_> fo;
+  __shared__ Folds<TS::X, TS::Y, TS::Z> fo;
   __shared__ uint64_t bar;
-  species_tile<P, M>(g, f, nspec, Origin{(int)blockIdx.x * SX_, (int)blockIdx.y * SY_, (int)blockIdx.z * SZ_}, sm,
-                     fo, zd, &bar, &tm);
+  species_tile<P, M, true, false, TS>(
+      g, f, nspec, Origin{(int)blockIdx.x * TS::X, (int)blockIdx.y * TS::Y, (int)blockIdx.z * TS::Z}, sm, fo, zd, &bar,
+      &tm);
 }
-template <bool P, int M>
-__global__ void __launch_bounds__(SX_* SY_, SENGA_SPECRK_MINB)
+template <bool P, int M, class TS = Tile3>
+__global__ void __launch_bounds__(TS::X* TS::Y, SENGA_SPECRK_MINB * 256 / (TS::X * TS::Y))
     k_species_rk_t(Geo g, Fields f, int nspec, RK rk, ZDec zd, const __grid_constant__ RkMaps tm) {
   extern __shared__ __align__(128) double sm[];
-  __shared__ Folds<SX_, SY_, SZ_> fo;
+  __shared__ Folds<TS::X, TS::Y, TS::Z> fo;
   __shared__ uint64_t bar;
-  species_rk_tile<P, M>(g, f, nspec, rk,
-                        Origin{(int)blockIdx.x * SX_, (int)blockIdx.y * SY_, (int)blockIdx.z * SZ_}, sm, fo, zd,
-                        &bar, &tm);
+  species_rk_tile<P, M, true, false, TS>(
+      g, f, nspec, rk, Origin{(int)blockIdx.x * TS::X, (int)blockIdx.y * TS::Y, (int)blockIdx.z * TS::Z}, sm, fo, zd,
+      &bar, &tm);
+}
+
+// ---- boxes with one point in y and z: one warp per 32 points (Tile1) ----
+template <bool P>
+__global__ void __launch_bounds__(Tile1::X) k_flow_line(Geo g, Fields f) {
+  __shared__ double sm[kLineSmem];
+  __shared__ Folds<Tile1::X, 1, 1> fo;
+  flow_tile<P, false, true, Tile1>(g, f, Origin{(int)blockIdx.x * Tile1::X, 0, 0}, sm, fo, ZDec{});
+}
+template <bool P>
+__global__ void __launch_bounds__(Tile1::X) k_species_line(Geo g, Fields f, int nspec) {
+  __shared__ double sm[kLineSmem];
+  __shared__ Folds<Tile1::X, 1, 1> fo;
+  species_tile<P, 0, true, false, Tile1>(g, f, nspec, Origin{(int)blockIdx.x * Tile1::X, 0, 0}, sm, fo, ZDec{});
+}
+template <bool P>
+__global__ void __launch_bounds__(Tile1::X) k_species_rk_line(Geo g, Fields f, int nspec, RK rk) {
+  __shared__ double sm[kLineSmem];
+  __shared__ Folds<Tile1::X, 1, 1> fo;
+  species_rk_tile<P, 0, true, false, Tile1>(g, f, nspec, rk, Origin{(int)blockIdx.x * Tile1::X, 0, 0}, sm, fo, ZDec{});
 }
 
 // Species pass and species+RK pass of one tile in one CTA, for all-periodic
@@ -129,11 +152,32 @@ void set_attrs() {
     cudaFuncSetAttribute(k_species_rk_t<P, P ? 2 : 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          kSpecRkSmem * 8);
   }
+  cudaFuncSetAttribute(k_flow_t<P, false, TileS>, cudaFuncAttributeMaxDynamicSharedMemorySize, flow_smem<TileS> * 8);
+  cudaFuncSetAttribute(k_flow_t<P, P, TileS>, cudaFuncAttributeMaxDynamicSharedMemorySize, flow_smem<TileS> * 8);
+  cudaFuncSetAttribute(k_species_t<P, 0, TileS>, cudaFuncAttributeMaxDynamicSharedMemorySize, spec_smem<TileS> * 8);
+  cudaFuncSetAttribute(k_species_rk_t<P, 0, TileS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       spec_rk_smem<TileS> * 8);
   cudaFuncSetAttribute(k_flow_b<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFlowSmem * 8);
   cudaFuncSetAttribute(k_species_b<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSpecSmem * 8);
   cudaFuncSetAttribute(k_species_rk_b<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSpecRkSmem * 8);
   done[dev] = true;
 }
+
+// 1D runs (a z split has more than one plane)
+bool one_line(const Geo& g, const ZDec& zd) { return g.ny == 1 && g.nz == 1 && zd.nr <= 1; }
+unsigned line_tiles(const Geo& g) { return (unsigned)((g.nx + Tile1::X - 1) / Tile1::X); }
+
+// Boxes of so few tiles that SMs stay idle take the smaller ones (TileS): at
+// 32^3 (64 tiles, 128 small ones) flow 44.5 -> 32.9, species of the 9-species
+// mechanism 33.9 -> 23.5, species+RK 17.1 -> 9.6 us; once every SM has a tile,
+// the smaller tile only stages more halo per point.
+constexpr int64_t kSmallTiles = 148;
+bool small_tiles(const Geo& g) {
+  const dim3 t = tiles(g, FX, FY, FZ);
+  return (int64_t)t.x * t.y * t.z <= kSmallTiles;
+}
+dim3 tiles_s(const Geo& g) { return tiles(g, TileS::X, TileS::Y, TileS::Z); }
+constexpr int kThreadsS = TileS::X * TileS::Y;
 
 bool all_periodic(const Geo& g) { return g.per[0] && g.per[1] && g.per[2]; }
 
@@ -201,21 +245,36 @@ bool make_map(CUtensorMap* m, const double* base, const Geo& g, int nk, unsigned
 }  // namespace
 
 void launch_flow(const Geo& g, const Fields& f, int, cudaStream_t s, const ZDec& zd) {
+  if (one_line(g, zd)) {
+    if (g.per[0]) k_flow_line<true><<<line_tiles(g), Tile1::X, 0, s>>>(g, f);
+    else k_flow_line<false><<<line_tiles(g), Tile1::X, 0, s>>>(g, f);
+    return;
+  }
+  const bool small = small_tiles(g);
   if (all_periodic(g)) {
     set_attrs<true>();
-    if (stage_mode(g, f, zd, KFlow) == 1)
-      k_flow_t<true, true><<<tiles(g, FX, FY, FZ), FX * FY, kFlowSmem * 8, s>>>(g, f, zd);
-    else
-      k_flow_t<true, false><<<tiles(g, FX, FY, FZ), FX * FY, kFlowSmem * 8, s>>>(g, f, zd);
+    if (stage_mode(g, f, zd, KFlow) == 1) {
+      if (small) k_flow_t<true, true, TileS><<<tiles_s(g), kThreadsS, flow_smem<TileS> * 8, s>>>(g, f, zd);
+      else k_flow_t<true, true><<<tiles(g, FX, FY, FZ), FX * FY, kFlowSmem * 8, s>>>(g, f, zd);
+    } else {
+      if (small) k_flow_t<true, false, TileS><<<tiles_s(g), kThreadsS, flow_smem<TileS> * 8, s>>>(g, f, zd);
+      else k_flow_t<true, false><<<tiles(g, FX, FY, FZ), FX * FY, kFlowSmem * 8, s>>>(g, f, zd);
+    }
   } else {
     set_attrs<false>();
-    k_flow_t<false, false><<<tiles(g, FX, FY, FZ), FX * FY, kFlowSmem * 8, s>>>(g, f, zd);
+    if (small) k_flow_t<false, false, TileS><<<tiles_s(g), kThreadsS, flow_smem<TileS> * 8, s>>>(g, f, zd);
+    else k_flow_t<false, false><<<tiles(g, FX, FY, FZ), FX * FY, kFlowSmem * 8, s>>>(g, f, zd);
   }
 }
 
 void launch_species_a(const Geo& g, const Fields& f, int nspec, cudaStream_t s, const ZDec& zd) {
   if (species_mma_ok(g, f, zd)) {
     launch_species_mma(g, f, nspec, s);
+    return;
+  }
+  if (one_line(g, zd)) {
+    if (g.per[0]) k_species_line<true><<<line_tiles(g), Tile1::X, 0, s>>>(g, f, nspec);
+    else k_species_line<false><<<line_tiles(g), Tile1::X, 0, s>>>(g, f, nspec);
     return;
   }
   const dim3 grid = tiles(g, SX_, SY_, SZ_);
@@ -231,10 +290,14 @@ void launch_species_a(const Geo& g, const Fields& f, int nspec, cudaStream_t s, 
       m = 1;
     if (m == 2) k_species_t<true, 2><<<grid, SX_ * SY_, kSpecSmem * 8, s>>>(g, f, nspec, zd, tm);
     else if (m == 1) k_species_t<true, 1><<<grid, SX_ * SY_, kSpecSmem * 8, s>>>(g, f, nspec, zd, tm);
+    else if (small_tiles(g))
+      k_species_t<true, 0, TileS><<<tiles_s(g), kThreadsS, spec_smem<TileS> * 8, s>>>(g, f, nspec, zd, tm);
     else k_species_t<true, 0><<<grid, SX_ * SY_, kSpecSmem * 8, s>>>(g, f, nspec, zd, tm);
   } else {
     set_attrs<false>();
-    k_species_t<false, 0><<<grid, SX_ * SY_, kSpecSmem * 8, s>>>(g, f, nspec, zd, tm);
+    if (small_tiles(g))
+      k_species_t<false, 0, TileS><<<tiles_s(g), kThreadsS, spec_smem<TileS> * 8, s>>>(g, f, nspec, zd, tm);
+    else k_species_t<false, 0><<<grid, SX_ * SY_, kSpecSmem * 8, s>>>(g, f, nspec, zd, tm);
   }
 }
 
@@ -264,6 +327,11 @@ void launch_species_b_rk(const Geo& g, const Fields& f, int nspec, const RK& rk,
     const char* e = getenv("SENGA_SPECRK");
     if (e && std::string(e) == "z" && launch_species_b_rk_z(g, f, nspec, rk, s, zd)) return;
   }
+  if (one_line(g, zd)) {
+    if (g.per[0]) k_species_rk_line<true><<<line_tiles(g), Tile1::X, 0, s>>>(g, f, nspec, rk);
+    else k_species_rk_line<false><<<line_tiles(g), Tile1::X, 0, s>>>(g, f, nspec, rk);
+    return;
+  }
   const dim3 grid = tiles(g, SX_, SY_, SZ_);
   RkMaps tm{};
   if (all_periodic(g)) {
@@ -274,10 +342,14 @@ void launch_species_b_rk(const Geo& g, const Fields& f, int nspec, const RK& rk,
       m = 1;
     if (m == 2) k_species_rk_t<true, 2><<<grid, SX_ * SY_, kSpecRkSmem * 8, s>>>(g, f, nspec, rk, zd, tm);
     else if (m == 1) k_species_rk_t<true, 1><<<grid, SX_ * SY_, kSpecRkSmem * 8, s>>>(g, f, nspec, rk, zd, tm);
+    else if (small_tiles(g))
+      k_species_rk_t<true, 0, TileS><<<tiles_s(g), kThreadsS, spec_rk_smem<TileS> * 8, s>>>(g, f, nspec, rk, zd, tm);
     else k_species_rk_t<true, 0><<<grid, SX_ * SY_, kSpecRkSmem * 8, s>>>(g, f, nspec, rk, zd, tm);
   } else {
     set_attrs<false>();
-    k_species_rk_t<false, 0><<<grid, SX_ * SY_, kSpecRkSmem * 8, s>>>(g, f, nspec, rk, zd, tm);
+    if (small_tiles(g))
+      k_species_rk_t<false, 0, TileS><<<tiles_s(g), kThreadsS, spec_rk_smem<TileS> * 8, s>>>(g, f, nspec, rk, zd, tm);
+    else k_species_rk_t<false, 0><<<grid, SX_ * SY_, kSpecRkSmem * 8, s>>>(g, f, nspec, rk, zd, tm);
   }
 }
 

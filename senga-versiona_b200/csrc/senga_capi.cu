@@ -713,11 +713,15 @@ int senga_set_transport(senga_ctx* c, int mixw, int mixp, int soret, int dufour,
     }
     const int64_t n = c->geo.n;
     const int nb = m.w + m.p + m.t;
-    const int64_t fields = 1 + 5 * (int64_t)nb + (m.tdr ? c->nspec : 0);
+    const int64_t fields = 1 + m.p + 5 * (int64_t)nb + (m.tdr ? c->nspec : 0);
     CK(cudaMalloc(&c->mixt_pool, (size_t)(fields * n) * sizeof(double)));
     double* p = c->mixt_pool;
     m.wmix = p;
     p += n;
+    if (m.p) {
+      m.owmix = p;
+      p += n;
+    }
     const int on[3] = {m.w, m.p, m.t};
     for (int b = 0; b < 3; ++b) {
       if (!on[b]) continue;

@@ -156,9 +156,12 @@ constexpr unsigned kStatusPersistTimeout = 16u;
 // tables bit for bit (select_mech). SENGA_MECH=generic in the environment
 // forces the table-driven kernel.
 int select_mech(const senga_chem& chem, const senga_diff& diff);
-// Returns the number of kernels it launched (the long mechanisms run as two).
+// Returns the number of kernels it launched (one to three).
 int launch_thermo(const Geo& g, const Fields& f, const senga_chem* dchem, const senga_diff* ddiff, int nspec,
                   int flmavt, int mech, cudaStream_t s);
+// the table-driven form of any mechanism of more than two species
+int launch_thermo_tables(const Geo& g, const Fields& f, const senga_chem* dchem, const senga_diff* ddiff, int nspec,
+                         int flmavt, cudaStream_t s);
 void launch_flow(const Geo& g, const Fields& f, int nspec, cudaStream_t s, const ZDec& zd = ZDec{});
 void launch_species_a(const Geo& g, const Fields& f, int nspec, cudaStream_t s, const ZDec& zd = ZDec{});
 void launch_species_b_rk(const Geo& g, const Fields& f, int nspec, const RK& rk, cudaStream_t s,
@@ -252,6 +255,7 @@ struct MixtParams {
   int w, p, t;
   unsigned sor, duf, tdr;
   double* wmix;      // [n]
+  double* owmix;     // [n] 1 / W_mix, nullptr without the pressure terms
   double* lng[3];    // [n] each, nullptr when off
   double* g1[3];     // [3][n] first derivatives
   double* g2[3];     // [n] sum of second derivatives (x part zeroed on diffusion-flux faces)

@@ -44,27 +44,86 @@ constexpr int SX_ = SENGA_TILE_X, SY_ = SENGA_TILE_Y, SZ_ = 2;
 constexpr int SNW = SX_ * SY_ / 32;
 static_assert(FX * FY == 256 && SX_ * SY_ == 256, "the stencil kernels run 256 threads per tile");
 
+// Tile of a kernel: its shape and buffer types. Tile3 for every box; Tile1 for
+// boxes with one point in y and z, one warp a tile. A 1D flame of 1001 points
+// filled 32 blocks in which 15 of 16 threads held no point, 18 x 12 copies of
+// the one line were staged and every y and z difference formed (species 58,
+// flow 48, species+RK 29 us a launch; 16, 8 and 14 us on these tiles).
+struct Tile3 {
+  static constexpr bool kLine = false;
+  static constexpr int X = FX, Y = FY, Z = FZ;
+  using Star = tile::Star<X, Y, Z>;
+  using Box = tile::Box<X, Y, Z>;
+  using XRow = tile::XRow<X, Y, Z>;
+  using YRow = tile::YRow<X, Y, Z>;
+  using ZCol = tile::ZCol<X, Y, Z>;
+  using Slab = tile::Slab<X, Y, Z>;
+  using Col = Column<Z>;
+};
+struct Tile1 {
+  static constexpr bool kLine = true;
+  static constexpr int X = 32, Y = 1, Z = 1;
+  using Star = Line<X>;
+  using Box = Line<X>;
+  using XRow = Line<X>;
+  using YRow = Line<X>;
+  using ZCol = Line<X>;
+  using Slab = Line<X>;
+  using Col = PointColumn;
+};
+// Tile3 for boxes of fewer tiles than SMs: the same plane of points, half the
+// planes or rows, so that twice the CTAs share the work of a box that leaves
+// SMs idle (kernels_tiled.cu: small_tiles).
+#ifndef SENGA_SMALL_Y
+#define SENGA_SMALL_Y 8
+#endif
+#ifndef SENGA_SMALL_Z
+#define SENGA_SMALL_Z 1
+#endif
+struct TileS {
+  static constexpr bool kLine = false;
+  static constexpr int X = FX, Y = SENGA_SMALL_Y, Z = SENGA_SMALL_Z;
+  using Star = tile::Star<X, Y, Z>;
+  using Box = tile::Box<X, Y, Z>;
+  using XRow = tile::XRow<X, Y, Z>;
+  using YRow = tile::YRow<X, Y, Z>;
+  using ZCol = tile::ZCol<X, Y, Z>;
+  using Slab = tile::Slab<X, Y, Z>;
+  using Col = Column<Z>;
+};
+constexpr int cmax(int a, int b) { return a > b ? a : b; }
+// dynamic shared memory of the kernels on a tile (doubles)
+template <class TS>
+constexpr int flow_smem = cmax(cmax(TS::XRow::SIZE + TS::YRow::SIZE + TS::ZCol::SIZE + TS::Star::SIZE,
+                                    2 * TS::Star::SIZE),
+                               cmax(3 * TS::XRow::SIZE + 3 * TS::YRow::SIZE, TS::Star::SIZE + TS::Box::SIZE));
+// species: the slabs, then the rho w z-columns, one per thread, [k][thread]
+template <class TS>
+constexpr int spec_smem = TS::XRow::SIZE + TS::YRow::SIZE + 3 * TS::Slab::SIZE + (TS::Z + 2 * H) * TS::X * TS::Y;
+// species+RK: two slabs, then the prefetched S register and rate of the next
+// species' own points, double-buffered: [buffer][run | rate][z][thread]
+template <class TS>
+constexpr int spec_rk_smem = 2 * TS::Slab::SIZE + 4 * TS::Z * TS::X * TS::Y;
+
+// shared memory of a Tile1 tile (doubles): the flow kernel's six rows; the
+// species kernels' five lines and prefetched values fit too
+constexpr int kLineSmem = 8 * Line<Tile1::X>::SIZE;
+
 using FStar = Star<FX, FY, FZ>;
 using FBox = Box<FX, FY, FZ>;
 using FXRow = XRow<FX, FY, FZ>;
 using FYRow = YRow<FX, FY, FZ>;
 using FZCol = ZCol<FX, FY, FZ>;
 
-constexpr int cmax(int a, int b) { return a > b ? a : b; }
-constexpr int kFlowSmem = cmax(cmax(FXRow::SIZE + FYRow::SIZE + FZCol::SIZE + FStar::SIZE, 2 * FStar::SIZE),
-                                cmax(3 * FXRow::SIZE + 3 * FYRow::SIZE, FStar::SIZE + FBox::SIZE));
+constexpr int kFlowSmem = flow_smem<Tile3>;
 
 using SSlab = Slab<SX_, SY_, SZ_>;
 using SXRow = XRow<SX_, SY_, SZ_>;
 using SYRow = YRow<SX_, SY_, SZ_>;
 using SCol = Column<SZ_>;
-// the species kernel's rho w z-columns: one per thread, [k][thread]
 constexpr int kSpecColW = (SZ_ + 2 * H) * SX_ * SY_;
-constexpr int kSpecSmem = SXRow::SIZE + SYRow::SIZE + 3 * SSlab::SIZE + kSpecColW;
-// species+RK: two slabs, then the prefetched S register and rate of the next
-// species' own points, double-buffered: [buffer][run | rate][z][thread]
-constexpr int kRkPre = 2 * SZ_ * SX_ * SY_;
-constexpr int kSpecRkSmem = 2 * SSlab::SIZE + 2 * kRkPre;
+constexpr int kSpecSmem = spec_smem<Tile3>;
+constexpr int kSpecRkSmem = spec_rk_smem<Tile3>;
 
 // Staging of a plain field: bulk copies on the TMA engine (B) or per-element
 // cp.async; and the wait for the group staged last (B: one mbarrier phase of
@@ -104,9 +163,15 @@ __device__ __forceinline__ bool sync_staged(BulkBar& bb, unsigned bytes, unsigne
   return false;
 }
 
-template <bool P, bool B = false, bool NC = true>
+template <bool P, bool B = false, bool NC = true, class TS = Tile3>
 __device__ __forceinline__ void flow_tile(const Geo& g, const Fields& f, const Origin o, double* sm,
-                                          Folds<FX, FY, FZ>& fo, const ZDec& zd, uint64_t* bar = nullptr) {
+                                          Folds<TS::X, TS::Y, TS::Z>& fo, const ZDec& zd, uint64_t* bar = nullptr) {
+  constexpr int FX = TS::X, FY = TS::Y, FZ = TS::Z, FNW = FX * FY / 32;
+  using FStar = typename TS::Star;
+  using FBox = typename TS::Box;
+  using FXRow = typename TS::XRow;
+  using FYRow = typename TS::YRow;
+  using FZCol = typename TS::ZCol;
   const int tx = threadIdx.x % FX, ty = threadIdx.x / FX;
   fo.init(g, o, zd);
   BulkBar bb{bar, 0u};
@@ -229,7 +294,7 @@ __device__ __forceinline__ void flow_tile(const Geo& g, const Fields& f, const O
       b = m * v;                 // rho v v
       c = m * ldf<NC>(pw + q);   // rho v w
     });
-    Column<FZ> cw, cm;
+    typename TS::Col cw, cm;
     cw.load(fo, tx, ty, LdT<NC>{f.vel + 2 * n});
     cm.load(fo, tx, ty, LdT<NC>{U + n});
     tile_sync();
@@ -474,11 +539,17 @@ constexpr int kCarryRate = kFuseMaxSpec * SZ_ * SX_ * SY_;  // doubles of shared
 
 // M: 0 per-element cp.async, 1 bulk row copies, 2 one tensor copy per buffer
 // for tiles away from the wrap (bulk rows for the others)
-template <bool P, int M = 0, bool NC = true, bool KEEP = false>
+template <bool P, int M = 0, bool NC = true, bool KEEP = false, class TS = Tile3>
 __device__ __forceinline__ void species_tile(const Geo& g, const Fields& f, int nspec, const Origin o, double* sm,
-                                             Folds<SX_, SY_, SZ_>& fo, const ZDec& zd, uint64_t* bar = nullptr,
+                                             Folds<TS::X, TS::Y, TS::Z>& fo, const ZDec& zd, uint64_t* bar = nullptr,
                                              const SpecMaps* tm = nullptr, SpecCarry* carry = nullptr) {
+  constexpr int SX_ = TS::X, SY_ = TS::Y, SZ_ = TS::Z, SNW = SX_ * SY_ / 32;
+  using SXRow = typename TS::XRow;
+  using SYRow = typename TS::YRow;
+  using SSlab = typename TS::Slab;
+  using SCol = typename TS::Col;
   constexpr bool B = M > 0;
+  constexpr bool WREG = KEEP || TS::kLine;  // the rho w column in registers
   const bool tens = M == 2 && tensor_tile<SX_, SY_, SZ_>(g, o, sm);
   constexpr unsigned kSlabT = 8u * SSlab::SIZE;  // a tensor copy fills the whole slab
   const unsigned slab_bytes = tens ? kSlabT : SSlab::kBulkBytes;
@@ -529,12 +600,12 @@ __device__ __forceinline__ void species_tile(const Geo& g, const Fields& f, int 
   double* const colw = sm + SXRow::SIZE + SYRow::SIZE + 3 * SSlab::SIZE;
   SCol rwc;
   rwc.load(fo, tx, ty, LdT<NC>{rw});
-  if constexpr (!KEEP) {
+  if constexpr (!WREG) {
 #pragma unroll
     for (int k = 0; k < SZ_ + 2 * H; ++k) colw[k * (SX_ * SY_) + threadIdx.x] = rwc.c[k];
   }
   auto wcol = [&](int k) {
-    if constexpr (KEEP) return rwc.c[k];
+    if constexpr (WREG) return rwc.c[k];
     else return colw[k * (SX_ * SY_) + threadIdx.x];
   };
   double vcx[SZ_], vcy[SZ_], vcz[SZ_], vt[SZ_], rE[SZ_], dvm[SZ_];
@@ -566,51 +637,55 @@ __device__ __forceinline__ void species_tile(const Geo& g, const Fields& f, int 
         const double yq = cy.c[z + H];
         double r = w0[z];
         r = r - 0.5 * yq * dvm[z];
-        if constexpr (P) {
-          // all periodic: each staged neighbour of Y, rho u, rho v read once
-          // into registers and shared by the flux, first and second
-          // derivatives (same arithmetic as the generic path)
-          double d1px, d1py, d2x, d2y, uc, vc;
-          {
-            double yv[2 * H + 1], fv[2 * H + 1];
+        // each staged neighbour of Y, rho u, rho v read once into registers and
+        // shared by the flux, first and second derivatives
+        double d1px, d1py, dyx, dyy, d2x, d2y, uc, vc;
+        {
+          double yv[2 * H + 1], fv[2 * H + 1];
 #pragma unroll
-            for (int m = 0; m <= 2 * H; ++m) {
-              yv[m] = bS.v(t.x + m - H, t.y, t.z);
-              fv[m] = bru.v(t.x + m - H, t.y, t.z);
-            }
-            d1px = d1core([&](int m) { return yv[m + H] * fv[m + H]; }, t.gx, g.nx, 1) * g.ovd[0];
-            yx[z] = d1core([&](int m) { return yv[m + H]; }, t.gx, g.nx, 1) * g.ovd[0];
-            d2x = d2core([&](int m) { return yv[m + H]; }, t.gx, g.nx, 1) * g.ovd2[0];
-            uc = fv[H];
+          for (int m = 0; m <= 2 * H; ++m) {
+            yv[m] = bS.v(t.x + m - H, t.y, t.z);
+            fv[m] = bru.v(t.x + m - H, t.y, t.z);
           }
-          {
-            double yv[2 * H + 1], fv[2 * H + 1];
-#pragma unroll
-            for (int m = 0; m <= 2 * H; ++m) {
-              yv[m] = bS.v(t.x, t.y + m - H, t.z);
-              fv[m] = brv.v(t.x, t.y + m - H, t.z);
-            }
-            d1py = d1core([&](int m) { return yv[m + H] * fv[m + H]; }, t.gy, g.ny, 1) * g.ovd[1];
-            yy[z] = d1core([&](int m) { return yv[m + H]; }, t.gy, g.ny, 1) * g.ovd[1];
-            d2y = d2core([&](int m) { return yv[m + H]; }, t.gy, g.ny, 1) * g.ovd2[1];
-            vc = fv[H];
-          }
-          r = r - 0.5 * (d1px + d1py + d1core([&](int m) { return cy.c[t.z + H + m] * wcol(t.z + H + m); }, t.gz, g.nz, 1) * g.ovd[2]);
-          yz[z] = d1z<P>(g, t, cy);
-          r = r - 0.5 * (yx[z] * uc + yy[z] * vc + yz[z] * wcol(z + H));
-          rate[z] = r;
-          fn3[z] = d2x + d2y + d2z<P>(g, t, cy);  // Laplacian for now
-        } else {
-          r = r - 0.5 * (d1p<0, P>(g, t, bS, bru) + d1p<1, P>(g, t, bS, brv) + d1core([&](int m) { return cy.c[t.z + H + m] * wcol(t.z + H + m); }, t.gz, g.nz, 1) * g.ovd[2]);
-          yx[z] = d1<0, P>(g, t, bS);
-          yy[z] = d1<1, P>(g, t, bS);
-          yz[z] = d1z<P>(g, t, cy);
-          r = r - 0.5 * (yx[z] * bru.v(t.x, t.y, t.z) + yy[z] * brv.v(t.x, t.y, t.z) + yz[z] * wcol(z + H));
-          rate[z] = r;
-          // FxxDIF/FxxADB zero the x diffusive terms on the face plane (rhscal.f:1581-1955)
-          const bool dif = !P && (face_bits(g, t.gx) & BF_DIF);
-          fn3[z] = (dif ? 0.0 : d2<0, P>(g, t, bS)) + d2<1, P>(g, t, bS) + d2z<P>(g, t, cy);  // Laplacian for now
+          d1px = d1core([&](int m) { return yv[m + H] * fv[m + H]; }, t.gx, g.nx, 1);
+          dyx = d1core([&](int m) { return yv[m + H]; }, t.gx, g.nx, 1);
+          d2x = d2core([&](int m) { return yv[m + H]; }, t.gx, g.nx, 1);
+          uc = fv[H];
         }
+        const int e = P ? -1 : end_row(g, t.gx);
+        if (!P && e >= 0) {
+          auto y = [&](int m) { return bS.v(t.x + m, t.y, t.z); };
+          d1px = d1end([&](int m) { return bS.v(t.x + m, t.y, t.z) * bru.v(t.x + m, t.y, t.z); }, e);
+          dyx = d1end(y, e);
+          d2x = d2end(y, e);
+        }
+        if constexpr (TS::kLine) {
+          d1py = dyy = d2y = 0.0;
+          vc = brv.v(t.x, t.y, t.z);
+        } else {
+          double yv[2 * H + 1], fv[2 * H + 1];
+#pragma unroll
+          for (int m = 0; m <= 2 * H; ++m) {
+            yv[m] = bS.v(t.x, t.y + m - H, t.z);
+            fv[m] = brv.v(t.x, t.y + m - H, t.z);
+          }
+          d1py = d1core([&](int m) { return yv[m + H] * fv[m + H]; }, t.gy, g.ny, 1);
+          dyy = d1core([&](int m) { return yv[m + H]; }, t.gy, g.ny, 1);
+          d2y = d2core([&](int m) { return yv[m + H]; }, t.gy, g.ny, 1);
+          vc = fv[H];
+        }
+        yx[z] = dyx * g.ovd[0];
+        yy[z] = dyy * g.ovd[1];
+        double d1pz = 0.0;
+        if constexpr (!TS::kLine)
+          d1pz = d1core([&](int m) { return cy.c[t.z + H + m] * wcol(t.z + H + m); }, t.gz, g.nz, 1);
+        r = r - 0.5 * (d1px * g.ovd[0] + d1py * g.ovd[1] + d1pz * g.ovd[2]);
+        yz[z] = d1z<P>(g, t, cy);
+        r = r - 0.5 * (yx[z] * uc + yy[z] * vc + yz[z] * wcol(z + H));
+        rate[z] = r;
+        // FxxDIF/FxxADB zero the x diffusive terms on the face plane (rhscal.f:1581-1955)
+        const bool dif = !P && (face_bits(g, t.gx) & BF_DIF);
+        fn3[z] = (dif ? 0.0 : d2x * g.ovd2[0]) + d2y * g.ovd2[1] + d2z<P>(g, t, cy);  // Laplacian for now
       }
     }
     // rho D_k and h_k staged together (one barrier pair): correction
@@ -673,11 +748,15 @@ __device__ __forceinline__ void species_tile(const Geo& g, const Fields& f, int 
 }
 
 // -------------------------------------------------------------------------
-template <bool P, int M = 0, bool NC = true, bool KEEP = false>
+template <bool P, int M = 0, bool NC = true, bool KEEP = false, class TS = Tile3>
 __device__ __forceinline__ void species_rk_tile(const Geo& g, const Fields& f, int nspec, const RK& rk,
-                                                const Origin o, double* sm, Folds<SX_, SY_, SZ_>& fo,
+                                                const Origin o, double* sm, Folds<TS::X, TS::Y, TS::Z>& fo,
                                                 const ZDec& zd, uint64_t* bar = nullptr, const RkMaps* tm = nullptr,
                                                 const SpecCarry* carry = nullptr) {
+  constexpr int SX_ = TS::X, SY_ = TS::Y, SZ_ = TS::Z, SNW = SX_ * SY_ / 32;
+  using SSlab = typename TS::Slab;
+  using SCol = typename TS::Col;
+  constexpr int kRkPre = 2 * SZ_ * SX_ * SY_;
   constexpr bool B = M > 0;
   const bool tens = M == 2 && tensor_tile<SX_, SY_, SZ_>(g, o, sm);
   const unsigned slab_bytes = tens ? 8u * SSlab::SIZE : SSlab::kBulkBytes;

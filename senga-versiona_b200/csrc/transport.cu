@@ -51,6 +51,7 @@ __global__ void __launch_bounds__(kMixBlock) k_mixt_pre(Geo g, Fields f, MixtPar
   c3 = 1.0 / c3;
   const double wmix = f.uin[q] * c3;
   m.wmix[q] = wmix;
+  if (m.owmix) m.owmix[q] = 1.0 / wmix;
   const double T = f.t[q];
   if (m.w) m.lng[0][q] = log(wmix);
   if (m.p) m.lng[1][q] = log(f.p[q]);
@@ -72,22 +73,57 @@ __global__ void __launch_bounds__(kMixBlock) k_mixt_pre(Geo g, Fields f, MixtPar
   }
 }
 
-__global__ void __launch_bounds__(kMixBlock) k_mixt_grad(Geo g, MixtParams m) {
-  const int64_t q = (int64_t)blockIdx.x * kMixBlock + threadIdx.x;
-  if (q >= g.n) return;
+// Gradients of the logarithms on the species kernels' tiles: each field staged
+// once with its x and y halos, the z column in registers (one thread a point
+// over global memory re-folded every neighbour and switched over the closure
+// rows: 64 us on 64x56x48, 15 us so; 1001-point line 58 -> 4.4 us).
+constexpr int MX = 32, MY = 8, MZ = 2;
+struct MTile3 {
+  static constexpr bool kLine = false;
+  static constexpr int X = MX, Y = MY, Z = MZ;
+  using Slab = tile::Slab<X, Y, Z>;
+  using Col = tile::Column<Z>;
+};
+struct MTile1 {  // boxes with one point in y and z (tiles.cuh)
+  static constexpr bool kLine = true;
+  static constexpr int X = 32, Y = 1, Z = 1;
+  using Slab = tile::Line<X>;
+  using Col = tile::PointColumn;
+};
+
+template <bool P, class TS>
+__global__ void __launch_bounds__(TS::X* TS::Y) k_mixt_grad(Geo g, MixtParams m) {
+  using namespace tile;
+  using Slab = typename TS::Slab;
+  extern __shared__ double sm[];
+  __shared__ Folds<TS::X, TS::Y, TS::Z> fo;
+  const Origin o{(int)blockIdx.x * TS::X, (int)blockIdx.y * TS::Y, (int)blockIdx.z * TS::Z};
+  const int tx = threadIdx.x % TS::X, ty = threadIdx.x / TS::X;
+  fo.init(g, o);
+  tile_sync();
   const int64_t n = g.n;
-  const Pt pt = point_of(g, q);
-  const bool dif = !g.per[0] && (face_bits(g, pt.i) & BF_DIF);
-  const int on[3] = {m.w, m.p, m.t};
+  const double* const F[3] = {m.w ? m.lng[0] : nullptr, m.p ? m.lng[1] : nullptr, m.t ? m.lng[2] : nullptr};
 #pragma unroll
+  for (int b = 0; b < 3; ++b)
+    if (F[b]) Slab{sm + b * Slab::SIZE}.template stage<TS::X * TS::Y / 32>(fo, Ld{F[b]});
+  tile_sync();
+#pragma unroll 1
   for (int b = 0; b < 3; ++b) {
-    if (!on[b]) continue;
-    const Ld F{m.lng[b]};
-    m.g1[b][q] = D1<0>(g, pt, F);
-    m.g1[b][n + q] = D1<1>(g, pt, F);
-    m.g1[b][2 * n + q] = D1<2>(g, pt, F);
-    const double d2x = dif ? 0.0 : D2<0>(g, pt, F);
-    m.g2[b][q] = d2x + D2<1>(g, pt, F) + D2<2>(g, pt, F);
+    if (!F[b]) continue;
+    const Slab s{sm + b * Slab::SIZE};
+    typename TS::Col c;
+    c.load(fo, tx, ty, Ld{F[b]});
+#pragma unroll
+    for (int z = 0; z < TS::Z; ++z) {
+      const TP t = make_tp(g, o, tx, ty, z);
+      if (!t.valid) continue;
+      const bool dif = !P && (face_bits(g, t.gx) & BF_DIF);
+      m.g1[b][t.q] = d1<0, P>(g, t, s);
+      m.g1[b][n + t.q] = d1<1, P>(g, t, s);
+      m.g1[b][2 * n + t.q] = d1z<P>(g, t, c);
+      const double d2x = dif ? 0.0 : d2<0, P>(g, t, s);
+      m.g2[b][t.q] = d2x + d2<1, P>(g, t, s) + d2z<P>(g, t, c);
+    }
   }
 }
 
@@ -96,23 +132,22 @@ __global__ void __launch_bounds__(kMixBlock) k_mixt_grad(Geo g, MixtParams m) {
 // field a term differentiates is staged once per tile and species into a
 // shared-memory slab (x, y halos) plus a register column per thread (z
 // halo), the driving diffusivities as products formed while staging.
-constexpr int MX = 32, MY = 8, MZ = 2, MNW = MX * MY / 32;
-using MSlab = tile::Slab<MX, MY, MZ>;
-using MCol = tile::Column<MZ>;
-constexpr int kMixSmem = 3 * MSlab::SIZE;
-
 enum { kBrW = 0, kBrP = 1, kBrT = 2, kBrDufour = 3 };
 
 // DIFMIX * Y_k times a branch factor: 1 (molar mass), 1 - W_k/W_mix
-// (pressure), TDRMIX_k (Soret)
-template <int BR>
+// (pressure), TDRMIX_k (Soret). RECIP: x is 1/W_mix; a tile forms the factor
+// at its halo points too, nine times a point, and the divides made the
+// pressure branch 227 us against 124 us of the molar-mass one on 64x56x48
+// (147 us with the reciprocal).
+template <int BR, bool RECIP = false>
 struct DrivingF {
   const double* __restrict__ rd;
   const double* __restrict__ y;
-  const double* __restrict__ x;  // W_mix or TDRMIX_k
+  const double* __restrict__ x;  // W_mix (RECIP: 1/W_mix) or TDRMIX_k
   double wk;
   __device__ __forceinline__ double operator()(int64_t q) const {
     if (BR == kBrW) return rd[q] * y[q];
+    if (BR == kBrP && RECIP) return rd[q] * y[q] * (1.0 - wk * x[q]);
     if (BR == kBrP) return rd[q] * y[q] * (1.0 - wk / x[q]);
     return rd[q] * y[q] * x[q];
   }
@@ -139,10 +174,14 @@ struct DufF {
   __device__ __forceinline__ double operator()(int64_t q) const { return rg * t[q] * tk[q]; }
 };
 
-template <int BR, bool P>
-__global__ void __launch_bounds__(MX* MY, 2) k_mixt_species(Geo g, Fields f, MixtParams m,
-                                                            const senga_chem* __restrict__ ch, int nspec) {
+template <int BR, bool P, class TS>
+__global__ void __launch_bounds__(TS::X* TS::Y, TS::kLine ? 1 : 2) k_mixt_species(Geo g, Fields f, MixtParams m,
+                                                                                  const senga_chem* __restrict__ ch,
+                                                                                  int nspec) {
   using namespace tile;
+  constexpr int MX = TS::X, MY = TS::Y, MZ = TS::Z, MNW = MX * MY / 32;
+  using MSlab = typename TS::Slab;
+  using MCol = typename TS::Col;
   extern __shared__ double sm[];
   __shared__ Folds<MX, MY, MZ> fo;
   const Origin o{(int)blockIdx.x * MX, (int)blockIdx.y * MY, (int)blockIdx.z * MZ};
@@ -204,7 +243,8 @@ __global__ void __launch_bounds__(MX* MY, 2) k_mixt_species(Geo g, Fields f, Mix
       }
       continue;
     }
-    const DrivingF<BR> drv{rdk, yk, BR == kBrP ? m.wmix : tk, ch->wmolar[k]};
+    // (the lines keep the divide: few points, and no halo in y and z)
+    const DrivingF<BR, !TS::kLine> drv{rdk, yk, BR == kBrP ? (TS::kLine ? m.wmix : m.owmix) : tk, ch->wmolar[k]};
     // W, P: UTMP with the Dufour term; Soret: with it taken out again
     const EnthF en{hk, f.t, tk, rg, duf ? (BR == kBrT ? 2 : 1) : 0};
     MCol cA, cB;
@@ -283,15 +323,39 @@ __global__ void __launch_bounds__(kMixBlock) k_mixt_wall(Geo g, Fields f, MixtPa
   f.vtmp[q] = vt;
 }
 
+dim3 mix_tiles(const Geo& g) {
+  return dim3((unsigned)((g.nx + MX - 1) / MX), (unsigned)((g.ny + MY - 1) / MY), (unsigned)((g.nz + MZ - 1) / MZ));
+}
+void launch_grad(const Geo& g, const MixtParams& m, cudaStream_t s) {
+  const bool per = g.per[0] && g.per[1] && g.per[2];
+  if (g.ny == 1 && g.nz == 1) {
+    const unsigned grid = (unsigned)((g.nx + MTile1::X - 1) / MTile1::X);
+    constexpr int smem = 3 * MTile1::Slab::SIZE * 8;
+    if (per) k_mixt_grad<true, MTile1><<<grid, MTile1::X, smem, s>>>(g, m);
+    else k_mixt_grad<false, MTile1><<<grid, MTile1::X, smem, s>>>(g, m);
+  } else {
+    constexpr int smem = 3 * MTile3::Slab::SIZE * 8;
+    if (per) k_mixt_grad<true, MTile3><<<mix_tiles(g), MX * MY, smem, s>>>(g, m);
+    else k_mixt_grad<false, MTile3><<<mix_tiles(g), MX * MY, smem, s>>>(g, m);
+  }
+}
+
 // launches the branch's tile kernel and, with a wall, its wall terms;
 // returns the number of launches
 template <int BR>
 int launch_branch(const Geo& g, const Fields& f, const MixtParams& m, const senga_chem* dchem, int nspec,
                   cudaStream_t s) {
-  const dim3 grid((unsigned)((g.nx + MX - 1) / MX), (unsigned)((g.ny + MY - 1) / MY), (unsigned)((g.nz + MZ - 1) / MZ));
   const bool per = g.per[0] && g.per[1] && g.per[2];
-  if (per) k_mixt_species<BR, true><<<grid, MX * MY, kMixSmem * 8, s>>>(g, f, m, dchem, nspec);
-  else k_mixt_species<BR, false><<<grid, MX * MY, kMixSmem * 8, s>>>(g, f, m, dchem, nspec);
+  if (g.ny == 1 && g.nz == 1) {
+    const unsigned grid = (unsigned)((g.nx + MTile1::X - 1) / MTile1::X);
+    constexpr int smem = 3 * MTile1::Slab::SIZE * 8;
+    if (per) k_mixt_species<BR, true, MTile1><<<grid, MTile1::X, smem, s>>>(g, f, m, dchem, nspec);
+    else k_mixt_species<BR, false, MTile1><<<grid, MTile1::X, smem, s>>>(g, f, m, dchem, nspec);
+  } else {
+    constexpr int smem = 3 * MTile3::Slab::SIZE * 8;
+    if (per) k_mixt_species<BR, true, MTile3><<<mix_tiles(g), MX * MY, smem, s>>>(g, f, m, dchem, nspec);
+    else k_mixt_species<BR, false, MTile3><<<mix_tiles(g), MX * MY, smem, s>>>(g, f, m, dchem, nspec);
+  }
   if (BR == kBrDufour || !((g.bxl | g.bxr) & BF_WALL)) return 1;
   k_mixt_wall<BR == kBrDufour ? kBrW : BR>
       <<<dim3((unsigned)((g.ny * g.nz + kMixBlock - 1) / kMixBlock), 2), kMixBlock, 0, s>>>(g, f, m, dchem, nspec);
@@ -308,7 +372,7 @@ int launch_mixt(const Geo& g, const Fields& f, const MixtParams& m, const senga_
   k_mixt_pre<<<gr, kMixBlock, 0, s>>>(g, f, m, dchem, ddiff, nspec);
   int nl = 1;
   if (m.w || m.p || m.t) {
-    k_mixt_grad<<<gr, kMixBlock, 0, s>>>(g, m);
+    launch_grad(g, m, s);
     ++nl;
   }
   if (m.duf) nl += launch_branch<kBrDufour>(g, f, m, dchem, nspec, s);
