@@ -45,10 +45,15 @@ constexpr int kFaceBlock = 128;
 // value m points along DIR from (i, j, k); y and z periodic, x bounded (the
 // closures read only inward points). A box split along z (zd.nr > 1) reads
 // the z neighbours from the slab that owns their plane.
+// c (within five points of [0, n)) folded into [0, n)
+__device__ __forceinline__ int wrap(int c, int n) {
+  if (n <= 5) return (c % n + n) % n;
+  return c < 0 ? c + n : (c >= n ? c - n : c);
+}
 template <int DIR>
 __device__ __forceinline__ double at(const Geo& g, const ZDec& zd, const double* a, int i, int j, int k, int m) {
   if (DIR == 0) i += m;
-  if (DIR == 1) j = ((j + m) % g.ny + g.ny) % g.ny;
+  if (DIR == 1) j = wrap(j + m, g.ny);
   int64_t base = 0;
   if (DIR == 2) {
     if (zd.nr > 1) {
@@ -57,25 +62,26 @@ __device__ __forceinline__ double at(const Geo& g, const ZDec& zd, const double*
       base = zd.base[r];
       k = zg - r * g.nz;
     } else {
-      k = ((k + m) % g.nz + g.nz) % g.nz;
+      k = wrap(k + m, g.nz);
     }
   }
   return a[base + (int64_t)i + (int64_t)g.nx * (j + (int64_t)g.ny * k)];
 }
+// Derivative of (a - c0) along DIR; c0 = 0 (exact) for every field but the
+// pressure, whose gradient RHSVEL takes of p - p(1,1,1) (src/rhsvel.f:730-752).
+// A function, not inlined: a face kernel of a few warps runs its code once and
+// waits for the instructions, and with some 30 inlined copies of the closures
+// that wait was the kernel (23 us for the two points of a 1D box, 15 us so).
+template <int DIR>
+__device__ __noinline__ double dd_sub(const Geo& g, const ZDec& zd, const double* a, double c0, int i, int j, int k) {
+  const int c = DIR == 0 ? i : DIR == 1 ? j : k;
+  const int n = DIR == 0 ? g.nx : DIR == 1 ? g.ny : g.nz;
+  if (DIR == 1 ? n == 1 : DIR == 2 && n == 1 && zd.nr <= 1) return 0.0;  // differences of a point with itself
+  return d1core([&](int m) { return at<DIR>(g, zd, a, i, j, k, m) - c0; }, c, n, DIR == 0 ? g.per[0] : 1) * g.ovd[DIR];
+}
 template <int DIR>
 __device__ __forceinline__ double dd(const Geo& g, const ZDec& zd, const double* a, int i, int j, int k) {
-  const int c = DIR == 0 ? i : DIR == 1 ? j : k;
-  const int n = DIR == 0 ? g.nx : DIR == 1 ? g.ny : g.nz;
-  return d1core([&](int m) { return at<DIR>(g, zd, a, i, j, k, m); }, c, n, g.per[DIR]) * g.ovd[DIR];
-}
-// derivative of (a - c) along DIR: the pressure gradient of RHSVEL is taken of
-// p - p(1,1,1) (src/rhsvel.f:730-752)
-template <int DIR>
-__device__ __forceinline__ double dd_sub(const Geo& g, const ZDec& zd, const double* a, double c0, int i, int j,
-                                         int k) {
-  const int c = DIR == 0 ? i : DIR == 1 ? j : k;
-  const int n = DIR == 0 ? g.nx : DIR == 1 ? g.ny : g.nz;
-  return d1core([&](int m) { return at<DIR>(g, zd, a, i, j, k, m) - c0; }, c, n, g.per[DIR]) * g.ovd[DIR];
+  return dd_sub<DIR>(g, zd, a, 0.0, i, j, k);
 }
 
 // h_k(T) per unit mass of interval `it` (AMASCH polynomial, boundt.f:316-324)
@@ -189,8 +195,9 @@ __global__ void __launch_bounds__(kFaceBlock)
   }
 }
 
-__global__ void __launch_bounds__(kFaceBlock) k_face(Geo g, Fields f, NscbcParams bc, int nspec, const senga_chem* chem,
-                                                   ZDec zd) {
+__global__ void __launch_bounds__(kFaceBlock)
+    k_face(const __grid_constant__ Geo g, Fields f, NscbcParams bc, int nspec, const senga_chem* __restrict__ chem,
+           const __grid_constant__ ZDec zd) {
   const int nyz = g.ny * g.nz;
   const int jk = blockIdx.x * kFaceBlock + threadIdx.x;
   const int side = blockIdx.y;  // 0: x-left, 1: x-right
@@ -452,26 +459,37 @@ __global__ void __launch_bounds__(kFaceBlock) k_face(Geo g, Fields f, NscbcParam
 // fourth-order x derivative at the wall of rho D_k dY_k/dx over the wall and
 // the four planes inward, added to species k's rate and to VTMP (its energy
 // part is dropped: BOUNDS zeroes the wall's energy RHS).
-__global__ void __launch_bounds__(kFaceBlock) k_wall_flux(Geo g, Fields f, NscbcParams bc, int nspec) {
-  const int jk = blockIdx.x * kFaceBlock + threadIdx.x;
-  const int side = blockIdx.y;
+// One thread per wall point and species (threadIdx.y), the species' parts of
+// VTMP summed in species order through shared memory: with the species in a
+// loop of one thread the chain of loads was the kernel (23 us for 2 x 2560
+// points of 9 species, 10.3 us so).
+constexpr int kWallX = 32;  // wall points a block
+__global__ void __launch_bounds__(kWallX* SENGA_NSPCMX)
+    k_wall_flux(const __grid_constant__ Geo g, Fields f, NscbcParams bc, int nspec, const __grid_constant__ ZDec zd) {
+  __shared__ double part[SENGA_NSPCMX][kWallX];
+  const int jk = blockIdx.x * kWallX + threadIdx.x;
+  const int side = blockIdx.y, s = threadIdx.y;
   const int kind = side == 0 ? bc.xl : bc.xr;
-  if (jk >= g.ny * g.nz || (kind != 31 && kind != 32)) return;
-  const int j = jk % g.ny, k = jk / g.ny;
+  if (kind != 31 && kind != 32) return;  // the whole block
+  const bool in = jk < g.ny * g.nz;
   const int i = side == 0 ? 0 : g.nx - 1, st = side == 0 ? 1 : -1;
   const int64_t n = g.n, q = (int64_t)i + (int64_t)g.nx * jk;
-  const double c0 = (double)(25.0f / 12.0f), c3 = (double)(4.0f / 3.0f);  // single-precision literals as coded
-  double vt = f.vtmp[q];
-  for (int s = 0; s < nspec; ++s) {
+  if (in) {
+    const int j = jk % g.ny, k = jk / g.ny;
+    const double c0 = (double)(25.0f / 12.0f), c3 = (double)(4.0f / 3.0f);  // single-precision literals as coded
     double fv[5];
 #pragma unroll
     for (int m = 0; m < 5; ++m)
-      fv[m] = f.rd[s * n + q + m * st] * dd<0>(g, ZDec{}, f.y + s * n, i + m * st, j, k);  // x only: own slab
+      fv[m] = f.rd[s * n + q + m * st] * dd<0>(g, zd, f.y + s * n, i + m * st, j, k);  // x only: own slab
     const double w = side == 0 ? ((-c0) * fv[0] + 4.0 * fv[1] - 3.0 * fv[2] + c3 * fv[3] - 0.25 * fv[4]) * g.ovd[0]
                                : (c0 * fv[0] - 4.0 * fv[1] + 3.0 * fv[2] - c3 * fv[3] + 0.25 * fv[4]) * g.ovd[0];
     f.wdot[s * n + q] = f.wdot[s * n + q] + w;
-    vt = vt + w;
+    part[s][threadIdx.x] = w;
   }
+  __syncthreads();
+  if (!in || s != 0) return;
+  double vt = f.vtmp[q];
+  for (int k = 0; k < nspec; ++k) vt = vt + part[k][threadIdx.x];
   f.vtmp[q] = vt;
 }
 
@@ -481,28 +499,27 @@ __global__ void __launch_bounds__(kFaceBlock) k_wall_flux(Geo g, Fields f, Nscbc
 // fraction of the updated U register extrapolated with zero normal gradient,
 // Y_w = (12/25)(4 Y_1 - 3 Y_2 + (4/3) Y_3 - Y_4/4), clipped to [0, 1], times
 // the wall density, into both registers (lincom.f:171-210, fincom.f:171-210).
-__global__ void __launch_bounds__(kFaceBlock) k_wall_fix(Geo g, Fields f, NscbcParams bc, int nspec, int rk) {
-  const int jk = blockIdx.x * kFaceBlock + threadIdx.x;
-  const int side = blockIdx.y;
+// One thread per wall point and species, as k_wall_flux (13.6 -> 4.9 us).
+__global__ void __launch_bounds__(kWallX* SENGA_NSPCMX) k_wall_fix(Geo g, Fields f, NscbcParams bc, int rk) {
+  const int jk = blockIdx.x * kWallX + threadIdx.x;
+  const int side = blockIdx.y, s = threadIdx.y;
   const int kind = side == 0 ? bc.xl : bc.xr;
   if (jk >= g.ny * g.nz || (kind != 31 && kind != 32)) return;
   const int st = side == 0 ? 1 : -1;
   const int64_t n = g.n, q = (side == 0 ? 0 : g.nx - 1) + (int64_t)g.nx * jk;
-  if (kind == 31) f.t[q] = wall_t(f.t, q, st);
+  if (kind == 31 && s == 0) f.t[q] = wall_t(f.t, q, st);
   if (!rk) return;
   const double* U = f.uout;
   const double c1 = (double)(12.0f / 25.0f), c3 = (double)(4.0f / 3.0f);
-  for (int s = 0; s < nspec; ++s) {
-    const double* y = U + (5 + s) * n;
-    const double t1 = y[q + st] / U[q + st], t2 = y[q + 2 * st] / U[q + 2 * st];
-    const double t3 = y[q + 3 * st] / U[q + 3 * st], t4 = y[q + 4 * st] / U[q + 4 * st];
-    double yw = c1 * (4.0 * t1 - 3.0 * t2 + c3 * t3 - (0.25 * t4));
-    yw = fmin(1.0, yw);
-    yw = fmax(0.0, yw);
-    yw = U[q] * yw;
-    f.run[(5 + s) * n + q] = yw;
-    f.uout[(5 + s) * n + q] = yw;
-  }
+  const double* y = U + (5 + s) * n;
+  const double t1 = y[q + st] / U[q + st], t2 = y[q + 2 * st] / U[q + 2 * st];
+  const double t3 = y[q + 3 * st] / U[q + 3 * st], t4 = y[q + 4 * st] / U[q + 4 * st];
+  double yw = c1 * (4.0 * t1 - 3.0 * t2 + c3 * t3 - (0.25 * t4));
+  yw = fmin(1.0, yw);
+  yw = fmax(0.0, yw);
+  yw = U[q] * yw;
+  f.run[(5 + s) * n + q] = yw;
+  f.uout[(5 + s) * n + q] = yw;
 }
 
 }  // namespace
@@ -520,13 +537,13 @@ void launch_boundt(const Geo& g, const Fields& f, const NscbcParams& bc, int nsp
 void launch_wall_flux(const Geo& g, const Fields& f, const NscbcParams& bc, int nspec, cudaStream_t s) {
   if (!has_wall(bc)) return;
   const int nyz = g.ny * g.nz;
-  k_wall_flux<<<dim3((nyz + kFaceBlock - 1) / kFaceBlock, 2), kFaceBlock, 0, s>>>(g, f, bc, nspec);
+  k_wall_flux<<<dim3((nyz + kWallX - 1) / kWallX, 2), dim3(kWallX, nspec), 0, s>>>(g, f, bc, nspec, ZDec{});
 }
 
 void launch_wall_fix(const Geo& g, const Fields& f, const NscbcParams& bc, int nspec, bool rk, cudaStream_t s) {
   if (!has_wall(bc)) return;
   const int nyz = g.ny * g.nz;
-  k_wall_fix<<<dim3((nyz + kFaceBlock - 1) / kFaceBlock, 2), kFaceBlock, 0, s>>>(g, f, bc, nspec, rk ? 1 : 0);
+  k_wall_fix<<<dim3((nyz + kWallX - 1) / kWallX, 2), dim3(kWallX, nspec), 0, s>>>(g, f, bc, rk ? 1 : 0);
 }
 
 void launch_face(const Geo& g, const Fields& f, const NscbcParams& bc, int nspec, const senga_chem* dchem,
