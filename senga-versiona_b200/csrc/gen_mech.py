@@ -16,6 +16,7 @@ Usage: python gen_mech.py <out.cuh>
 """
 import math
 import os
+import struct
 import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -317,6 +318,7 @@ def gen(tag, c, d):
     w(f"struct Mech_{tag} {{")
     w(f"  static constexpr int NS = {ns};")
     w(f"  static constexpr bool MAVT = {'true' if mavt else 'false'};")
+    w("  static constexpr bool RECIP = true;")
     w("  __device__ __forceinline__ bool has(int) const { return true; }")
     w("  __device__ __forceinline__ int count() const { return NS; }")
     # ---- temper coefficients
@@ -549,7 +551,6 @@ def gen(tag, c, d):
             w(f"      double s1 = exp({f});")
         if c["mllist"][st] != 0:
             L = c["rclind"][c["mllist"][st] - 1]
-            import struct
             flc = struct.unpack("f", struct.pack("f", L[3]))[0]  # REAL (single) in the reference
             w(f"      {{ const double s4 = exp({h(L[0])} + {h(L[1])} * lnT - {h(L[2])} * ovT);")
             w("        const double pr = s3 * s4 / s1;")
@@ -635,6 +636,117 @@ def gen(tag, c, d):
     return "\n".join(o)
 
 
+def gen_ref(tag, c, d):
+    """The policy's transport and rates in the reference's own association:
+    one exp per polynomial and per rate, one divide per quotient. Contexts with
+    the adaptive time step run these: its error norm is a difference that
+    cancels all but the last digits of the state, so another rounding in the
+    thermochemistry shows up in the step size (1e-10 where the state agrees to
+    1e-14)."""
+    ns = c["nspec"]
+    o = []
+    w = o.append
+
+    def pick(it_var, a, b):
+        return a if a == b else f"({it_var} ? {b} : {a})"
+
+    w(f"struct Mech_{tag}_ref : Mech_{tag} {{")
+    w("  static constexpr bool RECIP = false;")
+    # ---- mixture-averaged transport
+    w("  __device__ __forceinline__ void mixture(double T, double p, double rho, const double (&ry)[NS], const double (&y)[NS], double& lam, double (&rd)[NS], double& mu) const {")
+    w(f"    const double lt = log(T / {h(d['tdifgb'])});")
+    w("    double c1 = 0.0, c2 = 0.0, c3 = 0.0;")
+    for s in range(ns):
+        w(f"    {{ const double lk = exp({poly_expr(d['condco'][s], 'lt')}); const double fm = ry[{s}] * {h(c['ovwmol'][s])};")
+        w("      c1 = c1 + fm * lk; c2 = c2 + fm / lk; c3 = c3 + fm; }")
+    w("    c3 = 1.0 / c3; c1 = c1 * c3; c2 = c2 * c3;")
+    w("    lam = 0.5 * (c1 + 1.0 / c2);")
+    w("    const double wmix = rho * c3;")
+    w(f"    const double povr = p / {h(d['pdifgb'])};")
+    # Wilke viscosity before the mixture diffusivities, so that the nine
+    # rho D_k are formed last and stored right after: the square roots
+    # and the diffusivity sums are never live together (fewer registers);
+    # mu_k is taken as sqrt(mu_k)^2 (within an ulp of mu_k)
+    for s in range(ns):
+        w(f"    const double sq{s} = sqrt(exp({poly_expr(d['viscco'][s], 'lt')})); const double rq{s} = 1.0 / sq{s};")
+    w("    mu = 0.0;")
+    for s in range(ns):
+        w("    { double cc = 0.0, fw;")
+        for t in range(ns):
+            w(f"      fw = 1.0 + sq{s} * rq{t} * {h(d['wilko2'][s][t])}; fw = {h(d['wilko1'][s][t])} * fw * fw; cc = cc + y[{t}] * {h(c['ovwmol'][t])} * fw;")
+        w(f"      mu = mu + y[{s}] * {h(c['ovwmol'][s])} * ((sq{s} * sq{s}) / cc); }}")
+    w("    double sumy = 0.0;")
+    for s in range(ns):
+        w(f"    sumy += y[{s}] + {h(DFCTOL)};")
+    for s in range(ns):
+        w(f"    double den{s} = 0.0;")
+    for s in range(ns):
+        for t in range(s + 1, ns):
+            w(f"    {{ const double inv = exp(-{poly_expr(d['diffco'][s][t], 'lt')}) * povr;")
+            w(f"      den{s} += (y[{t}] + {h(DFCTOL)}) * {h(c['ovwmol'][t])} * inv;")
+            w(f"      den{t} += (y[{s}] + {h(DFCTOL)}) * {h(c['ovwmol'][s])} * inv; }}")
+    for s in range(ns):
+        w(f"    rd[{s}] = rho * (sumy - (y[{s}] + {h(DFCTOL)})) / (den{s} * wmix);")
+    w("  }")
+    # ---- CHRATE
+    w("  __device__ __forceinline__ void chrate(double T, uint64_t itn, const double (&ry)[NS], double (&rate)[NS]) const {")
+    w("    const double lnT = log(T); const double ovT = 1.0 / T; (void)itn;")
+    for s in range(ns):
+        w(f"    rate[{s}] = 0.0;")
+    need_gibbs = c["ngibb"] > 0
+    if need_gibbs:
+        for s in range(ns):
+            np_, nh, nsy = c["ncpoly"][s][0], c["ncenth"][s][0], c["ncenpy"][s][0]
+            g0 = c["amolgb"][s][0]
+            g1 = c["amolgb"][s][1] if c["ntint"][s] > 1 else g0
+            w(f"    double gib{s}; {{ const int it = (itn >> {2 * s}) & 1; (void)it; double v = {pick('it', h(g0[np_ - 1]), h(g1[np_ - 1]))};")
+            for icp in range(np_ - 1, 0, -1):
+                w(f"      v = {pick('it', h(g0[icp - 1]), h(g1[icp - 1]))} + v * T;")
+            w(f"      gib{s} = {pick('it', h(g0[nh - 1]), h(g1[nh - 1]))} / T - {pick('it', h(g0[nsy - 1]), h(g1[nsy - 1]))} * lnT - v; }}")
+    w("    double s3 = 0.0; (void)s3;")
+    for st in range(c["nstep"]):
+        w(f"    {{ // step {st + 1}")
+        ib = c["mblist"][st]
+        flthrd = True
+        if ib != 0:
+            w("      s3 = 0.0;")
+            for s in range(ns):
+                w(f"      s3 += ry[{s}] * {h(c['ovwmol'][s] * c['effy3b'][ib - 1][s])};")
+        A, nexp, E = c["rparam"][st]
+        w(f"      double s2 = {h(A)} + {h(nexp)} * lnT - {h(E)} * ovT;")
+        w("      double s1 = exp(s2);")
+        if c["mllist"][st] != 0:
+            L = c["rclind"][c["mllist"][st] - 1]
+            flc = struct.unpack("f", struct.pack("f", L[3]))[0]  # REAL (single) in the reference
+            w(f"      {{ const double s4 = exp({h(L[0])} + {h(L[1])} * lnT - {h(L[2])} * ovT);")
+            w("        const double pr = s3 * s4 / s1;")
+            w(f"        s1 = s1 * ({h(flc)} * pr / (1.0 + pr)); s2 = log(s1); }}")
+            flthrd = False
+        for sp, _ in c["nrspec"][st]:
+            w(f"      s1 = s1 * fmax(ry[{sp - 1}] * {h(c['ovwmol'][sp - 1])}, 0.0);")
+        for sp, cf in c["nrcpec"][st]:
+            w(f"      {{ double fn = fmax(ry[{sp - 1}] * {h(c['ovwmol'][sp - 1])}, 1.0e-30); fn = exp({h(cf)} * log(fn)); s1 = s1 * (fn / (1.0 + 1.0e-15 * fn)); }}")
+        if c["mglist"][st] != 0:
+            for q, (sp, _) in enumerate(c["nsspec"][st]):
+                w(f"      s2 = s2 + {h(c['diffmu'][st][q])} * gib{sp - 1};")
+            w("      s2 = exp(s2);")
+            for sp, _ in c["npspec"][st]:
+                w(f"      s2 = s2 * fmax(ry[{sp - 1}] * {h(c['ovwmol'][sp - 1])}, 0.0);")
+            for sp, cf in c["npcpec"][st]:
+                w(f"      {{ double fn = fmax(ry[{sp - 1}] * {h(c['ovwmol'][sp - 1])}, 1.0e-30); fn = exp({h(cf)} * log(fn)); s2 = s2 * (fn / (1.0 + 1.0e-15 * fn)); }}")
+            w("      s1 = s1 - s2;")
+        else:
+            w("      (void)s2;")
+        if ib != 0 and flthrd:
+            w("      s1 = s1 * s3;")
+        for q, (sp, _) in enumerate(c["nsspec"][st]):
+            w(f"      rate[{sp - 1}] += s1 * {h(c['diffmw'][st][q])};")
+        w("    }")
+    w("  }")
+    w("};")
+    return "\n".join(o)
+
+
 def main():
     out = sys.argv[1] if len(sys.argv) > 1 else os.path.join(HERE, "mech_gen.cuh")
     parts = ["// GENERATED by gen_mech.py from ../data/*.dat -- do not edit.",
@@ -645,6 +757,7 @@ def main():
     ch2 = load_chem(os.path.join(DATA, "chem_h2.dat"))
     dh2 = load_diff(os.path.join(DATA, "diff_h2.dat"), ch2)
     parts.append(gen("h2", ch2, dh2))
+    parts.append(gen_ref("h2", ch2, dh2))
     parts += ["", "}  // namespace gen", "}  // namespace senga", ""]
     with open(out, "w") as fh:
         fh.write("\n".join(parts))

@@ -101,20 +101,21 @@ int launch_thermo(const Geo& g, const Fields& f, const senga_chem* dchem, const 
   if (mech == 1) {
     k_thermo<<<gr, kBlock, 0, s>>>(g, f, gen::Mech_onestep{});
   } else if (mech == 2) {
-    k_thermo_part<gen::Mech_h2, 1>
-        <<<(unsigned)((g.n + kPartBlock<1> - 1) / kPartBlock<1>), kPartBlock<1>, 0, s>>>(g, f, gen::Mech_h2{});
-    k_thermo_part<gen::Mech_h2, 2>
-        <<<(unsigned)((g.n + kPartBlock<2> - 1) / kPartBlock<2>), kPartBlock<2>, 0, s>>>(g, f, gen::Mech_h2{});
+    constexpr int b1 = kPartBlock<1>, b2 = kPartBlock<2>;
+    const unsigned g1 = (unsigned)((g.n + b1 - 1) / b1), g2 = (unsigned)((g.n + b2 - 1) / b2);
+    if (f.err) {  // adaptive time step: see Mech_h2_ref (gen_mech.py)
+      k_thermo_part<gen::Mech_h2_ref, 1><<<g1, b1, 0, s>>>(g, f, gen::Mech_h2_ref{});
+      k_thermo_part<gen::Mech_h2_ref, 2><<<g2, b2, 0, s>>>(g, f, gen::Mech_h2_ref{});
+    } else {
+      k_thermo_part<gen::Mech_h2, 1><<<g1, b1, 0, s>>>(g, f, gen::Mech_h2{});
+      k_thermo_part<gen::Mech_h2, 2><<<g2, b2, 0, s>>>(g, f, gen::Mech_h2{});
+    }
     return 2;
   } else if (nspec <= 2) {
     if (flmavt) k_thermo<<<gr, kBlock, 0, s>>>(g, f, MechTables<2, true>{dchem, ddiff, nspec});
     else k_thermo<<<gr, kBlock, 0, s>>>(g, f, MechTables<2, false>{dchem, ddiff, nspec});
-  } else if (nspec <= 9) {
-    if (flmavt) k_thermo<<<gr, kBlock, 0, s>>>(g, f, MechTables<9, true>{dchem, ddiff, nspec});
-    else k_thermo<<<gr, kBlock, 0, s>>>(g, f, MechTables<9, false>{dchem, ddiff, nspec});
-  } else {  // the reference's larger casefile mechanisms (16 and 18 species)
-    if (flmavt) k_thermo<<<gr, kBlock, 0, s>>>(g, f, MechTables<SENGA_NSPCMX, true>{dchem, ddiff, nspec});
-    else k_thermo<<<gr, kBlock, 0, s>>>(g, f, MechTables<SENGA_NSPCMX, false>{dchem, ddiff, nspec});
+  } else {
+    return launch_thermo_tables(g, f, dchem, ddiff, nspec, flmavt, s);
   }
   return 1;
 }

@@ -44,18 +44,30 @@ __device__ __forceinline__ double get_at(const double (&a)[NSM], int k) {
   return r;
 }
 
+// One thread's element of a [species][thread] array in shared memory: the
+// species array of the table-driven kernels (thermo_tables.cu), where an index
+// from a table is an address.
+constexpr int kTabBlock = 64;  // their threads a block: three arrays of 18 species are 27.6 KB, 8 blocks an SM
+struct SpArray {
+  double* p;
+  __device__ __forceinline__ double& operator[](int s) const { return p[s * kTabBlock]; }
+};
+__device__ __forceinline__ void add_at(const SpArray& a, int k, double v) { a[k] += v; }
+__device__ __forceinline__ double get_at(const SpArray& a, int k) { return a[k]; }
+
 // -------------------------------------------------------------------------
 // CHRATE for one point. ry: rho*Y_k, T, itn (updated interval index).
 // Gibbs functions and log T are hoisted out of the step loop: the reference
 // evaluates the same expressions per step, so the values are identical.
-template <int NSM>
-__device__ void chrate_point(const senga_chem* __restrict__ C, int nspec, const double (&ry)[NSM], double T,
-                             uint64_t itn, double (&rate)[NSM]) {
+// Arrays: registers of NSM species, or SpArray (NSM 0, nspec elements).
+template <int NSM, class RY, class GIB, class RATE>
+__device__ __forceinline__ void chrate_point(const senga_chem* __restrict__ C, int nspec, const RY& ry, double T,
+                                             uint64_t itn, GIB& gib, RATE& rate) {
   const double lnT = log(T);
   const double ovT = 1.0 / T;
-  double gib[NSM];
+  const int ns = NSM > 0 ? NSM : nspec;
 #pragma unroll
-  for (int s = 0; s < NSM; ++s) {
+  for (int s = 0; s < ns; ++s) {
     rate[s] = 0.0;
     gib[s] = 0.0;
     if (s < nspec && C->ngibb > 0) {
@@ -74,7 +86,7 @@ __device__ void chrate_point(const senga_chem* __restrict__ C, int nspec, const 
     if (ib != 0) {
       s3 = 0.0;
 #pragma unroll
-      for (int s = 0; s < NSM; ++s)
+      for (int s = 0; s < ns; ++s)
         if (s < nspec) s3 += ry[s] * (C->ovwmol[s] * C->effy3b[ib - 1][s]);
     }
     double s2 = C->rparam[st][0] + C->rparam[st][1] * lnT - C->rparam[st][2] * ovT;
@@ -159,6 +171,7 @@ template <int NSM, bool MAVT_>
 struct MechTables {
   static constexpr int NS = NSM;
   static constexpr bool MAVT = MAVT_;
+  static constexpr bool RECIP = false;
   const senga_chem* __restrict__ C;
   const senga_diff* __restrict__ Dt;
   int nspec;
@@ -291,7 +304,8 @@ struct MechTables {
     }
   }
   __device__ __forceinline__ void chrate(double T, uint64_t itn, const double (&ry)[NS], double (&rate)[NS]) const {
-    chrate_point<NS>(C, nspec, ry, T, itn, rate);
+    double gib[NS];
+    chrate_point<NS>(C, nspec, ry, T, itn, gib, rate);
   }
 };
 
@@ -319,8 +333,11 @@ __device__ __forceinline__ void thermo_point(const Geo& g, const Fields& f, cons
   const double rho = U[q], ru = U[n + q], rv = U[2 * n + q], rw = U[3 * n + q], re = U[4 * n + q];
 
   // ---- TEMPER: Newton inversion of e(T) from the previous T ----
-  const double orho = 1.0 / rho;  // one reciprocal for the 13 quotients by rho
-  const double ukuk = (ru * ru + rv * rv + rw * rw) * orho;
+  // quotients by rho: one reciprocal for all in the generated policies, a
+  // divide each in the table-driven one
+  const double orho = M::RECIP ? 1.0 / rho : 0.0;
+  auto by_rho = [&](double a) { return M::RECIP ? a * orho : a / rho; };
+  const double ukuk = by_rho(ru * ru + rv * rv + rw * rw);
   double tc[6], td[6];
   tc[0] = 0.5 * ukuk - re;
 #pragma unroll
@@ -352,7 +369,7 @@ __device__ __forceinline__ void thermo_point(const Geo& g, const Fields& f, cons
   uint64_t itn;
   double cpm;
   m.locate(T, ry, itn, cpm);
-  cpm = cpm * orho;
+  cpm = by_rho(cpm);
   const double p = T * rmix;
   f.t[q] = T;
   itn_store(f.itn, n, q, m.count(), itn);
@@ -366,18 +383,18 @@ __device__ __forceinline__ void thermo_point(const Geo& g, const Fields& f, cons
   double y[NS];
 #pragma unroll
   for (int s = 0; s < NS; ++s) {
-    y[s] = ry[s] * orho;
+    y[s] = by_rho(ry[s]);
     if (m.has(s)) f.y[s * n + q] = y[s];
   }
-  f.vel[q] = ru * orho;
-  f.vel[n + q] = rv * orho;
-  f.vel[2 * n + q] = rw * orho;
+  f.vel[q] = by_rho(ru);
+  f.vel[n + q] = by_rho(rv);
+  f.vel[2 * n + q] = by_rho(rw);
   if (f.mom) {
     f.mom[q] = ru;
     f.mom[n + q] = rv;
     f.mom[2 * n + q] = rw;
   }
-  f.e[q] = re * orho;
+  f.e[q] = by_rho(re);
 
   // ---- transport properties ----
   if (!M::MAVT) {
