@@ -1,7 +1,7 @@
 """Boxes with one point in y and z (one warp per 32 points), the closures of a
 bounded x direction where both ends fall into one tile or a tile ends at the
-boundary, and the table-driven thermochemistry over partial blocks: against
-the oracle, and bit for bit against what a box repeated in y and z gives.
+boundary, and the table-driven thermochemistry over partial blocks, against the
+oracle.
 
 Bound: 1e-10 of the field's maximum, as in the other parity tests."""
 import numpy as np
