@@ -250,18 +250,6 @@ __device__ __forceinline__ double dmcore_ends(const V2& v, int ea, bool ra_a, in
 // ---- global-memory forms (operator-level entry points) ----------------------
 // Periodic directions wrap the index; bounded ones never leave the domain
 // because the closures only read inward.
-template <int DIR, class F>
-__device__ __forceinline__ double D1(const Geo& g, const Pt& p, const F& f) {
-  const int n = ext<DIR>(g), c = crd<DIR>(p);
-  auto v = [&](int m) { return f(p.q + woff<DIR>(g, c, m)); };
-  return d1core(v, c, n, g.per[DIR]) * g.ovd[DIR];
-}
-template <int DIR, class F>
-__device__ __forceinline__ double D2(const Geo& g, const Pt& p, const F& f) {
-  const int n = ext<DIR>(g), c = crd<DIR>(p);
-  auto v = [&](int m) { return f(p.q + woff<DIR>(g, c, m)); };
-  return d2core(v, c, n, g.per[DIR]) * g.ovd2[DIR];
-}
 template <int DA, int DB, class F>
 __device__ __forceinline__ double DM(const Geo& g, const Pt& p, const F& f) {
   const int ca = crd<DA>(p), cb = crd<DB>(p);
