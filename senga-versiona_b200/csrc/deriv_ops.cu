@@ -11,10 +11,11 @@
 // its (x, y), with the in-plane neighbour offsets folded once into registers,
 // and the z operators slide a register window so that every value is loaded
 // (ZB + 10) / ZB times. One thread per point with a 64-bit index decode and
-// a fold per neighbour took 498 us for the nine operators on that field; this
-// form takes 281 us.
+// a fold per neighbour took 543 us of device time for the nine operators on
+// that field; this form takes 243 us (64^3: 57 and 45, 47x153x61: 85 and 59).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "senga_internal.h"
@@ -59,15 +60,22 @@ template <bool BIG>
 __device__ __forceinline__ int fold_off(int c, int m, int n, int st) {
   int cm = c + m;
   if (!BIG) {
-    while (cm < 0) cm += n;
-    while (cm >= n) cm -= n;
+    if (n > H) {
+      cm = cm < 0 ? cm + n : cm >= n ? cm - n : cm;
+    } else {
+      cm %= n;
+      if (cm < 0) cm += n;
+    }
   }
   return (cm - c) * st;
 }
 
-// x and y operators: ORD 1 or 2 along D (0 or 1)
+// x and y operators: ORD 1 or 2 along D (0 or 1). At four blocks an SM and one
+// plane a turn: two planes a turn took 76 registers, three blocks, and the
+// second y derivative 9.4 instead of 7.0 us on 80^3, 40 instead of 26 on
+// 192x160x120.
 template <bool BIG, int D, int ORD>
-__global__ void __launch_bounds__(kThreads) k_plane_op(Geo g, InLay il, int ntx, int zb, const double* __restrict__ in,
+__global__ void __launch_bounds__(kThreads, 4) k_plane_op(Geo g, InLay il, int ntx, int zb, const double* __restrict__ in,
                                                        double* __restrict__ out) {
   const Where w = where(g, ntx);
   if (!w.in) return;
@@ -82,7 +90,7 @@ __global__ void __launch_bounds__(kThreads) k_plane_op(Geo g, InLay il, int ntx,
   for (int64_t z0 = first_march() * zb; z0 < g.nz; z0 += march_step() * zb) {
     const int z1 = (int)(z0 + zb < g.nz ? z0 + zb : g.nz);
     if (g.per[D]) {
-#pragma unroll 2
+#pragma unroll 1
       for (int z = (int)z0; z < z1; ++z) {
         const double* const p = p0 + z * il.sz;
         auto v = [&](int m) { return __ldg(p + off[m + H]); };
@@ -116,6 +124,8 @@ __global__ void __launch_bounds__(kThreads) k_z_op(Geo g, InLay il, int ntx, con
         int z = (int)z0 + k - H;
         if (BIG) {  // past the last point's halo: unused
           z = z < g.nz + H ? z : g.nz + H - 1;
+        } else if (g.nz >= ZB + H) {  // one fold reaches every plane of the window
+          z = z < 0 ? z + g.nz : z >= g.nz ? z - g.nz : z;
         } else {
           z %= g.nz;
           if (z < 0) z += g.nz;
@@ -223,10 +233,10 @@ __global__ void __launch_bounds__(kThreads) k_mixed_ends(Geo g, InLay il, int ki
   out[q] = r * g.ovd[da] * g.ovd[db];
 }
 
-int pow2_at_least(int n, int most) {
-  int p = 1;
-  while (p < n && p < most) p *= 2;
-  return p;
+// n points in equal parts of at most `most`: the size of a part
+int even_part(int n, int most) {
+  const int parts = (n + most - 1) / most;
+  return (n + parts - 1) / parts;
 }
 
 template <bool BIG>
@@ -242,20 +252,28 @@ void launch(const Geo& g, int kind, const double* in, double* out, cudaStream_t 
     k_mixed_ends<BIG><<<(unsigned)((g.n + kThreads - 1) / kThreads), kThreads, 0, s>>>(g, il, kind, in, out);
     return;
   }
-  // 32 x 8 points of a plane per block where the box has them, wider or
-  // taller blocks on thin ones
-  int by = pow2_at_least(g.ny, 8), bx = pow2_at_least(g.nx, kThreads / by);
-  by = pow2_at_least(g.ny, kThreads / bx);
+  // About 32 x 8 points of a plane per block (wider or taller on thin boxes),
+  // in equal parts of the extents: a fixed 32 x 8 left a third of the threads
+  // of a 47 x 153 plane without a point. 16 x 16 where that fits and 32 does
+  // not: rows of whole warps (48^3: 30 us for the nine operators, 34 with 24
+  // points a row).
+  const int bx = even_part(g.nx, g.ny < 8 ? kThreads / g.ny : g.nx % 32 == 16 ? 16 : 32), by = even_part(g.ny, kThreads / bx);
   const int64_t ntx = (g.nx + bx - 1) / bx, nty = (g.ny + by - 1) / by;
-  // planes a thread marches over: as many as leave the chip 300 thousand
-  // threads (148 SMs x 2048)
+  // Planes a thread marches over: as many as leave the chip 75 thousand
+  // threads, a quarter of what it holds (148 SMs x 2048), twice that for the y
+  // operators, whose eleven rows come from L2 more than the others' values. A
+  // march of one plane spends its time on the folds: with marches that left
+  // 300 thousand threads, and fixed blocks, 80^3 took 112 us, 120x100x90 152;
+  // so 59 and 100 (one thread per point: 95 and 181).
   int zb = 1;
-  const int most = kind == 2 || kind == 5 ? kMaxZB : 8;
-  while (zb < most && g.n / (2 * zb) >= 300000) zb *= 2;
-  if (kind == 2 || kind == 5) zb = zb >= 16 ? 16 : zb >= 4 ? 4 : 1;
+  const bool zop = kind == 2 || kind == 5;
+  const int most = zop ? kMaxZB : 8;
+  const int64_t fewest = kind == 1 || kind == 4 ? 150000 : 75000;
+  while (zb < most && g.n / (2 * zb) >= fewest) zb *= 2;
+  if (zop) zb = zb >= 16 ? 16 : zb >= 4 ? 4 : 1;
   // and several marches per block where the plane is smaller than a block
   const int64_t nzb = (g.nz + zb - 1) / zb;
-  const int bz = pow2_at_least((int)(nzb < 64 ? nzb : 64), kThreads / (bx * by));
+  const int bz = (int)std::min<int64_t>({nzb, 64, kThreads / (bx * by)});
   const int64_t nzg = (nzb + bz - 1) / bz;
   const dim3 grid((unsigned)(ntx * nty), (unsigned)(nzg < 65535 ? nzg : 65535)), block(bx, by, bz);
   const size_t wb = (size_t)bz * (zb + 2 * H) * sizeof(int64_t);  // the z windows of a block
