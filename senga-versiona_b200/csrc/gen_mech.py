@@ -310,7 +310,186 @@ def groups_of(rows):
     return [(m[0], m) for m in seen.values()]
 
 
-def gen(tag, c, d):
+def gen_chrate_sum(c, w):
+    """CHRATE with one exp per rate, the exponents of a reverse rate added
+    before it: finite at every temperature at which the rate is."""
+    ns = c["nspec"]
+
+    def pick(it_var, a, b):
+        return a if a == b else f"({it_var} ? {b} : {a})"
+
+    w("  static __device__ __forceinline__ void chrate_sum(double T, uint64_t itn, const double (&ry)[NS], double (&rate)[NS]) {")
+    w("    const double lnT = log(T); const double ovT = 1.0 / T; (void)itn;")
+    for s in range(ns):
+        w(f"    rate[{s}] = 0.0;")
+    need_gibbs = c["ngibb"] > 0
+    if need_gibbs:
+        for s in range(ns):
+            np_, nh, nsy = c["ncpoly"][s][0], c["ncenth"][s][0], c["ncenpy"][s][0]
+            g0 = c["amolgb"][s][0]
+            g1 = c["amolgb"][s][1] if c["ntint"][s] > 1 else g0
+            w(f"    double gib{s}; {{ const int it = (itn >> {2 * s}) & 1; (void)it; double v = {pick('it', h(g0[np_ - 1]), h(g1[np_ - 1]))};")
+            for icp in range(np_ - 1, 0, -1):
+                w(f"      v = {pick('it', h(g0[icp - 1]), h(g1[icp - 1]))} + v * T;")
+            w(f"      gib{s} = {pick('it', h(g0[nh - 1]), h(g1[nh - 1]))} / T - {pick('it', h(g0[nsy - 1]), h(g1[nsy - 1]))} * lnT - v; }}")
+    w("    double s3 = 0.0; (void)s3;")
+    for st in range(c["nstep"]):
+        w(f"    {{ // step {st + 1}")
+        ib = c["mblist"][st]
+        flthrd = True
+        if ib != 0:
+            w("      s3 = 0.0;")
+            for s in range(ns):
+                w(f"      s3 += ry[{s}] * {h(c['ovwmol'][s] * c['effy3b'][ib - 1][s])};")
+        A, nexp, E = c["rparam"][st]
+        w(f"      double s2 = {h(A)} + {h(nexp)} * lnT - {h(E)} * ovT;")
+        w("      double s1 = exp(s2);")
+        if c["mllist"][st] != 0:
+            L = c["rclind"][c["mllist"][st] - 1]
+            flc = struct.unpack("f", struct.pack("f", L[3]))[0]  # REAL (single) in the reference
+            w(f"      {{ const double s4 = exp({h(L[0])} + {h(L[1])} * lnT - {h(L[2])} * ovT);")
+            w("        const double pr = s3 * s4 / s1;")
+            w(f"        s1 = s1 * ({h(flc)} * pr / (1.0 + pr)); s2 = log(s1); }}")
+            flthrd = False
+        for sp, _ in c["nrspec"][st]:
+            w(f"      s1 = s1 * fmax(ry[{sp - 1}] * {h(c['ovwmol'][sp - 1])}, 0.0);")
+        for sp, cf in c["nrcpec"][st]:
+            w(f"      {{ double fn = fmax(ry[{sp - 1}] * {h(c['ovwmol'][sp - 1])}, 1.0e-30); fn = exp({h(cf)} * log(fn)); s1 = s1 * (fn / (1.0 + 1.0e-15 * fn)); }}")
+        if c["mglist"][st] != 0:
+            for q, (sp, _) in enumerate(c["nsspec"][st]):
+                w(f"      s2 = s2 + {h(c['diffmu'][st][q])} * gib{sp - 1};")
+            w("      s2 = exp(s2);")
+            for sp, _ in c["npspec"][st]:
+                w(f"      s2 = s2 * fmax(ry[{sp - 1}] * {h(c['ovwmol'][sp - 1])}, 0.0);")
+            for sp, cf in c["npcpec"][st]:
+                w(f"      {{ double fn = fmax(ry[{sp - 1}] * {h(c['ovwmol'][sp - 1])}, 1.0e-30); fn = exp({h(cf)} * log(fn)); s2 = s2 * (fn / (1.0 + 1.0e-15 * fn)); }}")
+            w("      s1 = s1 - s2;")
+        else:
+            w("      (void)s2;")
+        if ib != 0 and flthrd:
+            w("      s1 = s1 * s3;")
+        for q, (sp, _) in enumerate(c["nsspec"][st]):
+            w(f"      rate[{sp - 1}] += s1 * {h(c['diffmw'][st][q])};")
+        w("    }")
+    w("  }")
+
+
+def gen_chrate_shared(c, w, need_gibbs, products):
+    """CHRATE with shared exps; reverse rates as products when `products`."""
+    ns = c["nspec"]
+    used = sorted({sp - 1 for st in range(c["nstep"]) if c["mglist"][st] for sp, _ in c["nsspec"][st]})
+    if need_gibbs:
+        # g_k of every species that a reversible step changes
+        w("  template <int IM>")
+        w("  __device__ __forceinline__ void gibbs_m(double T, double ovT, double lnT, uint64_t itn, double (&g)[NS]) const {")
+        for s in used:
+            np_, nh, nsy = c["ncpoly"][s][0], c["ncenth"][s][0], c["ncenpy"][s][0]
+            g0 = c["amolgb"][s][0]
+            g1 = c["amolgb"][s][1] if c["ntint"][s] > 1 else g0
+            w(f"    {{ const int it = (itn >> {2 * s}) & 1; (void)it; double v = {sel('it', h(g0[np_ - 1]), h(g1[np_ - 1]))};")
+            for icp in range(np_ - 1, 0, -1):
+                w(f"      v = {sel('it', h(g0[icp - 1]), h(g1[icp - 1]))} + v * T;")
+            w(f"      g[{s}] = {sel('it', h(g0[nh - 1]), h(g1[nh - 1]))} * ovT - {sel('it', h(g0[nsy - 1]), h(g1[nsy - 1]))} * lnT - v; }}")
+        w("  }")
+    w("  __device__ __forceinline__ void chrate(double T, uint64_t itn, const double (&ry)[NS], double (&rate)[NS]) const {")
+    w("    const double lnT = log(T); const double ovT = 1.0 / T; (void)itn; (void)lnT;")
+    for s in range(ns):
+        w(f"    rate[{s}] = 0.0;")
+    if need_gibbs:
+        w("    double gib[NS];")
+        w("    const int im = mode(itn);")
+        w("    if (im == 0) gibbs_m<0>(T, ovT, lnT, itn, gib);")
+        w("    else if (im == 1) gibbs_m<1>(T, ovT, lnT, itn, gib);")
+        w("    else gibbs_m<2>(T, ovT, lnT, itn, gib);")
+    if products:
+        # exp(sum dmu_k g_k) of a reverse rate as a product of exp(g_k) and
+        # their reciprocals: one exp per species instead of one per step (the
+        # exponents are small enough that every product stays in range)
+        for s in used:
+            w(f"    const double ep{s} = exp(gib[{s}]);")
+        neg = {sp - 1 for st in range(c["nstep"]) if c["mglist"][st] for q, (sp, _) in enumerate(c["nsspec"][st]) if c["diffmu"][st][q] < 0}
+        for s in sorted(neg):
+            w(f"    const double en{s} = 1.0 / ep{s};")
+    for s in sorted({sp - 1 for st in range(c["nstep"]) for key in ("nrspec", "npspec") for sp, _ in c[key][st]}):
+        w(f"    const double cm{s} = fmax(ry[{s}] * {h(c['ovwmol'][s])}, 0.0);")
+    # rate constants exp(A + n ln T - E / T): a literal where n = E = 0, powers
+    # of T for an integer n with E = 0, one exp(-E / T) shared by the steps of
+    # equal E and integer n, else its own exp
+    def power(n):
+        n = int(n)
+        return " * ".join(["T"] * n if n > 0 else ["ovT"] * -n)
+
+    small = lambda n: n == int(n) and abs(n) <= 3  # noqa: E731
+    esteps = {}
+    for st in range(c["nstep"]):
+        A, nexp, E = c["rparam"][st]
+        if E != 0.0 and small(nexp):
+            esteps.setdefault(E, []).append(st)
+    shared = {E: k for k, (E, sts) in enumerate(esteps.items()) if len(sts) > 1}
+    for E, k in shared.items():
+        w(f"    const double ee{k} = exp(-{h(E)} * ovT);")
+    w("    double s3 = 0.0; (void)s3;")
+    for st in range(c["nstep"]):
+        w(f"    {{ // step {st + 1}")
+        ib = c["mblist"][st]
+        flthrd = True
+        if ib != 0:
+            w("      s3 = 0.0;")
+            for s in range(ns):
+                w(f"      s3 += ry[{s}] * {h(c['ovwmol'][s] * c['effy3b'][ib - 1][s])};")
+        A, nexp, E = c["rparam"][st]
+        if E == 0.0 and small(nexp):
+            f = [h(math.exp(A))] + ([power(nexp)] if nexp else [])
+            w(f"      double s1 = {' * '.join(f)};")
+        elif E in shared and small(nexp):
+            f = [h(math.exp(A)), f"ee{shared[E]}"] + ([power(nexp)] if nexp else [])
+            w(f"      double s1 = {' * '.join(f)};")
+        else:
+            f = h(A) + (f" + {h(nexp)} * lnT" if nexp else "") + (f" - {h(E)} * ovT" if E else "")
+            w(f"      double s1 = exp({f});")
+        if c["mllist"][st] != 0:
+            L = c["rclind"][c["mllist"][st] - 1]
+            flc = struct.unpack("f", struct.pack("f", L[3]))[0]  # REAL (single) in the reference
+            w(f"      {{ const double s4 = exp({h(L[0])} + {h(L[1])} * lnT - {h(L[2])} * ovT);")
+            w("        const double pr = s3 * s4 / s1;")
+            w(f"        s1 = s1 * ({h(flc)} * pr / (1.0 + pr)); }}")
+            flthrd = False
+        if c["mglist"][st] != 0:
+            if products:
+                w("      double s2 = s1;")
+                for q, (sp, _) in enumerate(c["nsspec"][st]):
+                    dmu = int(c["diffmu"][st][q])
+                    for _ in range(abs(dmu)):
+                        w(f"      s2 = s2 * {'ep' if dmu > 0 else 'en'}{sp - 1};")
+            else:
+                w("      double s2 = log(s1);")
+                for q, (sp, _) in enumerate(c["nsspec"][st]):
+                    w(f"      s2 = s2 + {h(c['diffmu'][st][q])} * gib[{sp - 1}];")
+                w("      s2 = exp(s2);")
+        for sp, _ in c["nrspec"][st]:
+            w(f"      s1 = s1 * cm{sp - 1};")
+        for sp, cf in c["nrcpec"][st]:
+            w(f"      {{ double fn = fmax(ry[{sp - 1}] * {h(c['ovwmol'][sp - 1])}, 1.0e-30); fn = exp({h(cf)} * log(fn)); s1 = s1 * (fn / (1.0 + 1.0e-15 * fn)); }}")
+        if c["mglist"][st] != 0:
+            for sp, _ in c["npspec"][st]:
+                w(f"      s2 = s2 * cm{sp - 1};")
+            for sp, cf in c["npcpec"][st]:
+                w(f"      {{ double fn = fmax(ry[{sp - 1}] * {h(c['ovwmol'][sp - 1])}, 1.0e-30); fn = exp({h(cf)} * log(fn)); s2 = s2 * (fn / (1.0 + 1.0e-15 * fn)); }}")
+            w("      s1 = s1 - s2;")
+        if ib != 0 and flthrd:
+            w("      s1 = s1 * s3;")
+        for q, (sp, _) in enumerate(c["nsspec"][st]):
+            w(f"      rate[{sp - 1}] += s1 * {h(c['diffmw'][st][q])};")
+        w("    }")
+    w("  }")
+
+
+def gen(tag, c, d, shared=True):
+    """The policy of one mechanism. shared: exps and quotients shared (see
+    mixture and chrate below), interval-dependent functions in three modes, one
+    reciprocal of rho. Without it the plain forms: for short mechanisms, whose
+    kernel is bound by its loads and stores (the single-step one on
+    160x144x128: 97 us a launch plain, 104 us shared)."""
     ns = c["nspec"]
     mavt = d is not None
     o = []
@@ -318,7 +497,7 @@ def gen(tag, c, d):
     w(f"struct Mech_{tag} {{")
     w(f"  static constexpr int NS = {ns};")
     w(f"  static constexpr bool MAVT = {'true' if mavt else 'false'};")
-    w("  static constexpr bool RECIP = true;")
+    w(f"  static constexpr bool RECIP = {'true' if shared else 'false'};")
     w("  __device__ __forceinline__ bool has(int) const { return true; }")
     w("  __device__ __forceinline__ int count() const { return NS; }")
     # ---- temper coefficients
@@ -328,7 +507,10 @@ def gen(tag, c, d):
     # select and no second literal is left.
     allhi = sum(1 << (2 * s) for s in range(ns) if c["ntint"][s] > 1)
     w(f"  static constexpr uint64_t kAllHigh = {allhi}ull;")
-    w("  static __device__ __forceinline__ int mode(uint64_t itn) { return itn == 0 ? 0 : itn == kAllHigh ? 1 : 2; }")
+    if shared:
+        w("  static __device__ __forceinline__ int mode(uint64_t itn) { return itn == 0 ? 0 : itn == kAllHigh ? 1 : 2; }")
+    else:
+        w("  static __device__ __forceinline__ constexpr int mode(uint64_t) { return 2; }")
     w("  template <int IM>")
     w("  __device__ __forceinline__ void temper_coeffs_m(const double (&ry)[NS], uint64_t itn0, double (&tc)[6], double (&td)[6], double& rmix) const {")
     for s in range(ns):
@@ -477,113 +659,15 @@ def gen(tag, c, d):
         w(f"      hk[{s}] = {sel('it', h(a0[nh - 1]), h(a1[nh - 1]))} + v * T; }}")
     w("  }")
     # ---- CHRATE
+    gen_chrate_sum(c, w)
     need_gibbs = c["ngibb"] > 0
-    products = need_gibbs and gibbs_products_in_range(c)
-    used = sorted({sp - 1 for st in range(c["nstep"]) if c["mglist"][st] for sp, _ in c["nsspec"][st]})
-    if need_gibbs:
-        # g_k of every species that a reversible step changes
-        w("  template <int IM>")
-        w("  __device__ __forceinline__ void gibbs_m(double T, double ovT, double lnT, uint64_t itn, double (&g)[NS]) const {")
-        for s in used:
-            np_, nh, nsy = c["ncpoly"][s][0], c["ncenth"][s][0], c["ncenpy"][s][0]
-            g0 = c["amolgb"][s][0]
-            g1 = c["amolgb"][s][1] if c["ntint"][s] > 1 else g0
-            w(f"    {{ const int it = (itn >> {2 * s}) & 1; (void)it; double v = {sel('it', h(g0[np_ - 1]), h(g1[np_ - 1]))};")
-            for icp in range(np_ - 1, 0, -1):
-                w(f"      v = {sel('it', h(g0[icp - 1]), h(g1[icp - 1]))} + v * T;")
-            w(f"      g[{s}] = {sel('it', h(g0[nh - 1]), h(g1[nh - 1]))} * ovT - {sel('it', h(g0[nsy - 1]), h(g1[nsy - 1]))} * lnT - v; }}")
+    products = shared and need_gibbs and gibbs_products_in_range(c)
+    if not shared:
+        w("  __device__ __forceinline__ void chrate(double T, uint64_t itn, const double (&ry)[NS], double (&rate)[NS]) const {")
+        w("    chrate_sum(T, itn, ry, rate);")
         w("  }")
-    w("  __device__ __forceinline__ void chrate(double T, uint64_t itn, const double (&ry)[NS], double (&rate)[NS]) const {")
-    w("    const double lnT = log(T); const double ovT = 1.0 / T; (void)itn; (void)lnT;")
-    for s in range(ns):
-        w(f"    rate[{s}] = 0.0;")
-    if need_gibbs:
-        w("    double gib[NS];")
-        w("    const int im = mode(itn);")
-        w("    if (im == 0) gibbs_m<0>(T, ovT, lnT, itn, gib);")
-        w("    else if (im == 1) gibbs_m<1>(T, ovT, lnT, itn, gib);")
-        w("    else gibbs_m<2>(T, ovT, lnT, itn, gib);")
-    if products:
-        # exp(sum dmu_k g_k) of a reverse rate as a product of exp(g_k) and
-        # their reciprocals: one exp per species instead of one per step (the
-        # exponents are small enough that every product stays in range)
-        for s in used:
-            w(f"    const double ep{s} = exp(gib[{s}]);")
-        neg = {sp - 1 for st in range(c["nstep"]) if c["mglist"][st] for q, (sp, _) in enumerate(c["nsspec"][st]) if c["diffmu"][st][q] < 0}
-        for s in sorted(neg):
-            w(f"    const double en{s} = 1.0 / ep{s};")
-    for s in sorted({sp - 1 for st in range(c["nstep"]) for key in ("nrspec", "npspec") for sp, _ in c[key][st]}):
-        w(f"    const double cm{s} = fmax(ry[{s}] * {h(c['ovwmol'][s])}, 0.0);")
-    # rate constants exp(A + n ln T - E / T): a literal where n = E = 0, powers
-    # of T for an integer n with E = 0, one exp(-E / T) shared by the steps of
-    # equal E and integer n, else its own exp
-    def power(n):
-        n = int(n)
-        return " * ".join(["T"] * n if n > 0 else ["ovT"] * -n)
-
-    small = lambda n: n == int(n) and abs(n) <= 3  # noqa: E731
-    esteps = {}
-    for st in range(c["nstep"]):
-        A, nexp, E = c["rparam"][st]
-        if E != 0.0 and small(nexp):
-            esteps.setdefault(E, []).append(st)
-    shared = {E: k for k, (E, sts) in enumerate(esteps.items()) if len(sts) > 1}
-    for E, k in shared.items():
-        w(f"    const double ee{k} = exp(-{h(E)} * ovT);")
-    w("    double s3 = 0.0; (void)s3;")
-    for st in range(c["nstep"]):
-        w(f"    {{ // step {st + 1}")
-        ib = c["mblist"][st]
-        flthrd = True
-        if ib != 0:
-            w("      s3 = 0.0;")
-            for s in range(ns):
-                w(f"      s3 += ry[{s}] * {h(c['ovwmol'][s] * c['effy3b'][ib - 1][s])};")
-        A, nexp, E = c["rparam"][st]
-        if E == 0.0 and small(nexp):
-            f = [h(math.exp(A))] + ([power(nexp)] if nexp else [])
-            w(f"      double s1 = {' * '.join(f)};")
-        elif E in shared and small(nexp):
-            f = [h(math.exp(A)), f"ee{shared[E]}"] + ([power(nexp)] if nexp else [])
-            w(f"      double s1 = {' * '.join(f)};")
-        else:
-            f = h(A) + (f" + {h(nexp)} * lnT" if nexp else "") + (f" - {h(E)} * ovT" if E else "")
-            w(f"      double s1 = exp({f});")
-        if c["mllist"][st] != 0:
-            L = c["rclind"][c["mllist"][st] - 1]
-            flc = struct.unpack("f", struct.pack("f", L[3]))[0]  # REAL (single) in the reference
-            w(f"      {{ const double s4 = exp({h(L[0])} + {h(L[1])} * lnT - {h(L[2])} * ovT);")
-            w("        const double pr = s3 * s4 / s1;")
-            w(f"        s1 = s1 * ({h(flc)} * pr / (1.0 + pr)); }}")
-            flthrd = False
-        if c["mglist"][st] != 0:
-            if products:
-                w("      double s2 = s1;")
-                for q, (sp, _) in enumerate(c["nsspec"][st]):
-                    dmu = int(c["diffmu"][st][q])
-                    for _ in range(abs(dmu)):
-                        w(f"      s2 = s2 * {'ep' if dmu > 0 else 'en'}{sp - 1};")
-            else:
-                w("      double s2 = log(s1);")
-                for q, (sp, _) in enumerate(c["nsspec"][st]):
-                    w(f"      s2 = s2 + {h(c['diffmu'][st][q])} * gib[{sp - 1}];")
-                w("      s2 = exp(s2);")
-        for sp, _ in c["nrspec"][st]:
-            w(f"      s1 = s1 * cm{sp - 1};")
-        for sp, cf in c["nrcpec"][st]:
-            w(f"      {{ double fn = fmax(ry[{sp - 1}] * {h(c['ovwmol'][sp - 1])}, 1.0e-30); fn = exp({h(cf)} * log(fn)); s1 = s1 * (fn / (1.0 + 1.0e-15 * fn)); }}")
-        if c["mglist"][st] != 0:
-            for sp, _ in c["npspec"][st]:
-                w(f"      s2 = s2 * cm{sp - 1};")
-            for sp, cf in c["npcpec"][st]:
-                w(f"      {{ double fn = fmax(ry[{sp - 1}] * {h(c['ovwmol'][sp - 1])}, 1.0e-30); fn = exp({h(cf)} * log(fn)); s2 = s2 * (fn / (1.0 + 1.0e-15 * fn)); }}")
-            w("      s1 = s1 - s2;")
-        if ib != 0 and flthrd:
-            w("      s1 = s1 * s3;")
-        for q, (sp, _) in enumerate(c["nsspec"][st]):
-            w(f"      rate[{sp - 1}] += s1 * {h(c['diffmw'][st][q])};")
-        w("    }")
-    w("  }")
+    else:
+        gen_chrate_shared(c, w, need_gibbs, products)
     # ---- host-side exact match against the loaded tables
     w("  static bool matches(const senga_chem& C, const senga_diff& D) {")
     w("    bool ok = true;")
@@ -637,18 +721,15 @@ def gen(tag, c, d):
 
 
 def gen_ref(tag, c, d):
-    """The policy's transport and rates in the reference's own association:
-    one exp per polynomial and per rate, one divide per quotient. Contexts with
-    the adaptive time step run these: its error norm is a difference that
-    cancels all but the last digits of the state, so another rounding in the
-    thermochemistry shows up in the step size (1e-10 where the state agrees to
-    1e-14)."""
+    """The shared policy's transport and rates with nothing shared: one exp per
+    polynomial and per rate, one divide per quotient. Contexts with the adaptive
+    time step run these: its error norm is a difference that cancels all but the
+    last digits of the state, so another rounding in the thermochemistry shows
+    up in the step size (1e-10 to 3e-9 where the state agrees to 1e-14). The
+    plain policies need no such form."""
     ns = c["nspec"]
     o = []
     w = o.append
-
-    def pick(it_var, a, b):
-        return a if a == b else f"({it_var} ? {b} : {a})"
 
     w(f"struct Mech_{tag}_ref : Mech_{tag} {{")
     w("  static constexpr bool RECIP = false;")
@@ -688,60 +769,8 @@ def gen_ref(tag, c, d):
     for s in range(ns):
         w(f"    rd[{s}] = rho * (sumy - (y[{s}] + {h(DFCTOL)})) / (den{s} * wmix);")
     w("  }")
-    # ---- CHRATE
     w("  __device__ __forceinline__ void chrate(double T, uint64_t itn, const double (&ry)[NS], double (&rate)[NS]) const {")
-    w("    const double lnT = log(T); const double ovT = 1.0 / T; (void)itn;")
-    for s in range(ns):
-        w(f"    rate[{s}] = 0.0;")
-    need_gibbs = c["ngibb"] > 0
-    if need_gibbs:
-        for s in range(ns):
-            np_, nh, nsy = c["ncpoly"][s][0], c["ncenth"][s][0], c["ncenpy"][s][0]
-            g0 = c["amolgb"][s][0]
-            g1 = c["amolgb"][s][1] if c["ntint"][s] > 1 else g0
-            w(f"    double gib{s}; {{ const int it = (itn >> {2 * s}) & 1; (void)it; double v = {pick('it', h(g0[np_ - 1]), h(g1[np_ - 1]))};")
-            for icp in range(np_ - 1, 0, -1):
-                w(f"      v = {pick('it', h(g0[icp - 1]), h(g1[icp - 1]))} + v * T;")
-            w(f"      gib{s} = {pick('it', h(g0[nh - 1]), h(g1[nh - 1]))} / T - {pick('it', h(g0[nsy - 1]), h(g1[nsy - 1]))} * lnT - v; }}")
-    w("    double s3 = 0.0; (void)s3;")
-    for st in range(c["nstep"]):
-        w(f"    {{ // step {st + 1}")
-        ib = c["mblist"][st]
-        flthrd = True
-        if ib != 0:
-            w("      s3 = 0.0;")
-            for s in range(ns):
-                w(f"      s3 += ry[{s}] * {h(c['ovwmol'][s] * c['effy3b'][ib - 1][s])};")
-        A, nexp, E = c["rparam"][st]
-        w(f"      double s2 = {h(A)} + {h(nexp)} * lnT - {h(E)} * ovT;")
-        w("      double s1 = exp(s2);")
-        if c["mllist"][st] != 0:
-            L = c["rclind"][c["mllist"][st] - 1]
-            flc = struct.unpack("f", struct.pack("f", L[3]))[0]  # REAL (single) in the reference
-            w(f"      {{ const double s4 = exp({h(L[0])} + {h(L[1])} * lnT - {h(L[2])} * ovT);")
-            w("        const double pr = s3 * s4 / s1;")
-            w(f"        s1 = s1 * ({h(flc)} * pr / (1.0 + pr)); s2 = log(s1); }}")
-            flthrd = False
-        for sp, _ in c["nrspec"][st]:
-            w(f"      s1 = s1 * fmax(ry[{sp - 1}] * {h(c['ovwmol'][sp - 1])}, 0.0);")
-        for sp, cf in c["nrcpec"][st]:
-            w(f"      {{ double fn = fmax(ry[{sp - 1}] * {h(c['ovwmol'][sp - 1])}, 1.0e-30); fn = exp({h(cf)} * log(fn)); s1 = s1 * (fn / (1.0 + 1.0e-15 * fn)); }}")
-        if c["mglist"][st] != 0:
-            for q, (sp, _) in enumerate(c["nsspec"][st]):
-                w(f"      s2 = s2 + {h(c['diffmu'][st][q])} * gib{sp - 1};")
-            w("      s2 = exp(s2);")
-            for sp, _ in c["npspec"][st]:
-                w(f"      s2 = s2 * fmax(ry[{sp - 1}] * {h(c['ovwmol'][sp - 1])}, 0.0);")
-            for sp, cf in c["npcpec"][st]:
-                w(f"      {{ double fn = fmax(ry[{sp - 1}] * {h(c['ovwmol'][sp - 1])}, 1.0e-30); fn = exp({h(cf)} * log(fn)); s2 = s2 * (fn / (1.0 + 1.0e-15 * fn)); }}")
-            w("      s1 = s1 - s2;")
-        else:
-            w("      (void)s2;")
-        if ib != 0 and flthrd:
-            w("      s1 = s1 * s3;")
-        for q, (sp, _) in enumerate(c["nsspec"][st]):
-            w(f"      rate[{sp - 1}] += s1 * {h(c['diffmw'][st][q])};")
-        w("    }")
+    w("    chrate_sum(T, itn, ry, rate);")
     w("  }")
     w("};")
     return "\n".join(o)
@@ -753,7 +782,7 @@ def main():
              "// Straight-line thermochemistry policies (see gen_mech.py).",
              "#pragma once", "#include <cstdint>", '#include "senga_gpu.h"', "", "namespace senga {", "namespace gen {", ""]
     c1 = load_chem(os.path.join(DATA, "chem_1step.dat"))
-    parts.append(gen("onestep", c1, None))
+    parts.append(gen("onestep", c1, None, shared=False))
     ch2 = load_chem(os.path.join(DATA, "chem_h2.dat"))
     dh2 = load_diff(os.path.join(DATA, "diff_h2.dat"), ch2)
     parts.append(gen("h2", ch2, dh2))

@@ -333,8 +333,8 @@ __device__ __forceinline__ void thermo_point(const Geo& g, const Fields& f, cons
   const double rho = U[q], ru = U[n + q], rv = U[2 * n + q], rw = U[3 * n + q], re = U[4 * n + q];
 
   // ---- TEMPER: Newton inversion of e(T) from the previous T ----
-  // quotients by rho: one reciprocal for all in the generated policies, a
-  // divide each in the table-driven one
+  // quotients by rho: one reciprocal for all in the policies that share exps
+  // and quotients (gen_mech.py), a divide each in the others
   const double orho = M::RECIP ? 1.0 / rho : 0.0;
   auto by_rho = [&](double a) { return M::RECIP ? a * orho : a / rho; };
   const double ukuk = by_rho(ru * ru + rv * rv + rw * rw);
