@@ -268,11 +268,6 @@ def sel(it_var, a, b):
     return a if a == b else f"(IM == 0 ? {a} : IM == 1 ? {b} : {it_var} ? {b} : {a})"
 
 
-# Reverse rates as products of exp(Gibbs function) factors need every partial
-# product in range over these temperatures (the tables start at 300 K).
-GIB_T, GIB_LIMIT = (100.0, 200.0, 300.0, 1000.0, 3000.0, 6000.0), 650.0
-
-
 def gibbs(c, s, it, T):
     g = c["amolgb"][s][it]
     np_, nh, nsy = c["ncpoly"][s][it], c["ncenth"][s][it], c["ncenpy"][s][it]
@@ -282,22 +277,55 @@ def gibbs(c, s, it, T):
     return g[nh - 1] / T - g[nsy - 1] * math.log(T) - v
 
 
-def gibbs_products_in_range(c):
-    """True when every reverse rate can be formed from exp(g_k) factors: the
-    exponents of all factors and partial products, in the order in which they
-    are multiplied, stay below GIB_LIMIT in size (of 709)."""
+# Reverse rates as products of the forward rate constant and exp(Gibbs
+# function) factors: every factor and every partial product, in the order in
+# which they are multiplied, keeps an exponent of at most GIB_LIMIT in size
+# (exp is a normal number up to 708). Third-body sums of falloff steps are
+# taken between S3_MIN and S3_MAX kmol/m^3. The products serve the range of
+# temperatures around 300 to 3000 K where that holds.
+GIB_LIMIT, S3_MIN, S3_MAX = 650.0, 1.0e-12, 1.0e3
+
+
+def gibbs_products_fit(c, T):
+    """True when every reverse rate at T can be formed from exp(g_k) factors."""
+    lnT = math.log(T)
+    arrhenius = lambda r: r[0] + r[1] * lnT - r[2] / T  # noqa: E731
     for st in range(c["nstep"]):
         if not c["mglist"][st]:
             continue
-        for T in GIB_T:
-            total = 0.0
-            for q, (sp, _) in enumerate(c["nsspec"][st]):
-                d, s = c["diffmu"][st][q], sp - 1
-                it = 1 if c["ntint"][s] > 1 and T > c["tinthi"][s][0] else 0
-                total += d * gibbs(c, s, it, T)
-                if d != int(d) or max(abs(gibbs(c, s, it, T)), abs(total)) > GIB_LIMIT:
-                    return False
+        s1 = arrhenius(c["rparam"][st])
+        starts = [s1]
+        if c["mllist"][st]:  # s1 flc pr / (1 + pr), pr = s3 s4 / s1
+            L = c["rclind"][c["mllist"][st] - 1]
+            low = arrhenius(L) + math.log(L[3])
+            starts += [s1 + math.log(L[3]), low + math.log(S3_MIN), low + math.log(S3_MAX)]
+        sizes = list(starts)
+        total = 0.0
+        for q, (sp, _) in enumerate(c["nsspec"][st]):
+            d, s = c["diffmu"][st][q], sp - 1
+            if d != int(d):
+                return False
+            g = gibbs(c, s, 1 if c["ntint"][s] > 1 and T > c["tinthi"][s][0] else 0, T)
+            sizes.append(g)
+            for _ in range(abs(int(d))):
+                total += math.copysign(g, d * g)
+                sizes += [x + total for x in starts]
+        if max(abs(x) for x in sizes) > GIB_LIMIT:
+            return False
     return True
+
+
+def gibbs_product_range(c):
+    """(lowest, highest) temperature of the products, on a grid of 1%; None
+    when they do not hold from 300 to 3000 K."""
+    grid = [300.0 * 1.01 ** k for k in range(-400, 700)]
+    ok = [gibbs_products_fit(c, T) for T in grid]
+    lo = hi = 400
+    while lo > 0 and ok[lo - 1]:
+        lo -= 1
+    while hi + 1 < len(grid) and ok[hi + 1]:
+        hi += 1
+    return (grid[lo], grid[hi]) if ok[lo] and grid[hi] >= 3000.0 else None
 
 
 def groups_of(rows):
@@ -375,7 +403,8 @@ def gen_chrate_sum(c, w):
 
 
 def gen_chrate_shared(c, w, need_gibbs, products):
-    """CHRATE with shared exps; reverse rates as products when `products`."""
+    """CHRATE with shared exps; reverse rates as products, for the range of
+    temperatures `products` (chrate_fits; thermo_point takes chrate_sum outside)."""
     ns = c["nspec"]
     used = sorted({sp - 1 for st in range(c["nstep"]) if c["mglist"][st] for sp, _ in c["nsspec"][st]})
     if need_gibbs:
@@ -403,8 +432,7 @@ def gen_chrate_shared(c, w, need_gibbs, products):
         w("    else gibbs_m<2>(T, ovT, lnT, itn, gib);")
     if products:
         # exp(sum dmu_k g_k) of a reverse rate as a product of exp(g_k) and
-        # their reciprocals: one exp per species instead of one per step (the
-        # exponents are small enough that every product stays in range)
+        # their reciprocals: one exp per species instead of one per step
         for s in used:
             w(f"    const double ep{s} = exp(gib[{s}]);")
         neg = {sp - 1 for st in range(c["nstep"]) if c["mglist"][st] for q, (sp, _) in enumerate(c["nsspec"][st]) if c["diffmu"][st][q] < 0}
@@ -661,7 +689,9 @@ def gen(tag, c, d, shared=True):
     # ---- CHRATE
     gen_chrate_sum(c, w)
     need_gibbs = c["ngibb"] > 0
-    products = shared and need_gibbs and gibbs_products_in_range(c)
+    products = gibbs_product_range(c) if shared and need_gibbs else None
+    fits = f"T >= {h(products[0])} && T <= {h(products[1])}" if products else "true"  # NaN does not
+    w(f"  static __device__ __forceinline__ bool chrate_fits(double T) {{ (void)T; return {fits}; }}")
     if not shared:
         w("  __device__ __forceinline__ void chrate(double T, uint64_t itn, const double (&ry)[NS], double (&rate)[NS]) const {")
         w("    chrate_sum(T, itn, ry, rate);")
@@ -733,6 +763,7 @@ def gen_ref(tag, c, d):
 
     w(f"struct Mech_{tag}_ref : Mech_{tag} {{")
     w("  static constexpr bool RECIP = false;")
+    w("  static __device__ __forceinline__ bool chrate_fits(double) { return true; }")
     # ---- mixture-averaged transport
     w("  __device__ __forceinline__ void mixture(double T, double p, double rho, const double (&ry)[NS], const double (&y)[NS], double& lam, double (&rd)[NS], double& mu) const {")
     w(f"    const double lt = log(T / {h(d['tdifgb'])});")

@@ -303,11 +303,28 @@ struct MechTables {
       h[s] = ch[C->ncenth[s][it] - 1] + v * T;
     }
   }
+  static __device__ __forceinline__ bool chrate_fits(double) { return true; }
+  static __device__ __forceinline__ void chrate_sum(double, uint64_t, const double (&)[NS], double (&)[NS]) {}  // not called
   __device__ __forceinline__ void chrate(double T, uint64_t itn, const double (&ry)[NS], double (&rate)[NS]) const {
     double gib[NS];
     chrate_point<NS>(C, nspec, ry, T, itn, gib, rate);
   }
 };
+
+// CHRATE of a point outside the temperatures that a generated policy's
+// products of exps serve (gen_mech.py): exponents added, over what the
+// products gave. A function of its own, called when nothing else is left to
+// do: no state of a flame comes here, and a call in front of the products cost
+// them 536 B of spills a thread (part 2 on 128^3 25% slower).
+template <class M>
+__device__ __noinline__ void chrate_wide(const double* U, double* wdot, int64_t n, int64_t q, double T, uint64_t itn) {
+  double ry[M::NS], rate[M::NS];
+#pragma unroll
+  for (int s = 0; s < M::NS; ++s) ry[s] = U[(5 + s) * n + q];
+  M::chrate_sum(T, itn, ry, rate);
+#pragma unroll
+  for (int s = 0; s < M::NS; ++s) wdot[s * n + q] = rate[s];
+}
 
 // -------------------------------------------------------------------------
 // PART 0: everything; PART 1: all but CHRATE; PART 2: CHRATE only, from the
@@ -323,11 +340,14 @@ __device__ __forceinline__ void thermo_point(const Geo& g, const Fields& f, cons
 #pragma unroll
   for (int s = 0; s < NS; ++s) ry[s] = m.has(s) ? U[(5 + s) * n + q] : 0.0;
   if (PART == 2) {
+    const double T = f.t[q];
+    const uint64_t itn = itn_load(f, n, q, m.count());
     double rate[NS];
-    m.chrate(f.t[q], itn_load(f, n, q, m.count()), ry, rate);
+    m.chrate(T, itn, ry, rate);
 #pragma unroll
     for (int s = 0; s < NS; ++s)
       if (m.has(s)) f.wdot[s * n + q] = rate[s];
+    if (!M::chrate_fits(T)) chrate_wide<M>(U, f.wdot, n, q, f.t[q], itn_load(f, n, q, m.count()));
     return;
   }
   const double rho = U[q], ru = U[n + q], rv = U[2 * n + q], rw = U[3 * n + q], re = U[4 * n + q];
@@ -436,6 +456,7 @@ __device__ __forceinline__ void thermo_point(const Geo& g, const Fields& f, cons
 #pragma unroll
     for (int s = 0; s < NS; ++s)
       if (m.has(s)) f.wdot[s * n + q] = rate[s];
+    if (!M::chrate_fits(T)) chrate_wide<M>(U, f.wdot, n, q, f.t[q], itn_load(f, n, q, m.count()));
   }
 }
 
