@@ -167,17 +167,26 @@ void set_attrs() {
 bool one_line(const Geo& g, const ZDec& zd) { return g.ny == 1 && g.nz == 1 && zd.nr <= 1; }
 unsigned line_tiles(const Geo& g) { return (unsigned)((g.nx + Tile1::X - 1) / Tile1::X); }
 
-// Boxes of so few tiles that SMs stay idle take the smaller ones (TileS): at
-// 32^3 (64 tiles, 128 small ones) flow 44.5 -> 32.9, species of the 9-species
-// mechanism 33.9 -> 23.5, species+RK 17.1 -> 9.6 us; once every SM has a tile,
-// the smaller tile only stages more halo per point.
-constexpr int64_t kSmallTiles = 148;
-bool small_tiles(const Geo& g) {
-  const dim3 t = tiles(g, FX, FY, FZ);
-  return (int64_t)t.x * t.y * t.z <= kSmallTiles;
-}
 dim3 tiles_s(const Geo& g) { return tiles(g, TileS::X, TileS::Y, TileS::Z); }
 constexpr int kThreadsS = TileS::X * TileS::Y;
+constexpr int64_t kSms = 148;
+int64_t count(const dim3& t) { return (int64_t)t.x * t.y * t.z; }
+
+// Boxes of so few tiles that SMs stay idle take the smaller ones (TileS), which
+// stage more halo per point. Up to one large tile an SM that is a gain, also
+// where two small ones share an SM: each has half the points to go through.
+// Only the species kernel of periodic boxes, which stages five buffers a tile
+// and has no closures to evaluate, loses once small tiles share an SM. Large
+// against small tiles, us a launch, 9 species (in brackets 2):
+//   large tiles                   72           80           144
+//   flow, periodic            39.3  28.6   39.3  31.2   39.6  31.7 (39.7  31.8)
+//   flow, bounded x           50.1  30.4   50.1  40.6   50.8  41.9
+//   species+RK, periodic      20.3  10.9   20.3  15.5   21.0  16.3 ( 9.2   7.0)
+//   species+RK, bounded x     38.5  18.2   38.1  21.5   39.2  22.6
+//   species, periodic         32.9  23.1   33.0  34.7   33.6  35.7 (10.1  10.6)
+//   species, bounded x        50.6  31.7   51.2  46.2   51.5  47.4
+bool small_tiles(const Geo& g) { return count(tiles(g, FX, FY, FZ)) <= kSms; }
+bool small_species_tiles(const Geo& g) { return count(tiles_s(g)) <= kSms; }
 
 bool all_periodic(const Geo& g) { return g.per[0] && g.per[1] && g.per[2]; }
 
@@ -290,7 +299,7 @@ void launch_species_a(const Geo& g, const Fields& f, int nspec, cudaStream_t s, 
       m = 1;
     if (m == 2) k_species_t<true, 2><<<grid, SX_ * SY_, kSpecSmem * 8, s>>>(g, f, nspec, zd, tm);
     else if (m == 1) k_species_t<true, 1><<<grid, SX_ * SY_, kSpecSmem * 8, s>>>(g, f, nspec, zd, tm);
-    else if (small_tiles(g))
+    else if (small_species_tiles(g))
       k_species_t<true, 0, TileS><<<tiles_s(g), kThreadsS, spec_smem<TileS> * 8, s>>>(g, f, nspec, zd, tm);
     else k_species_t<true, 0><<<grid, SX_ * SY_, kSpecSmem * 8, s>>>(g, f, nspec, zd, tm);
   } else {
