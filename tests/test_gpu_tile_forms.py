@@ -1,8 +1,9 @@
 """Boxes on either side of the tile counts at which the stencil kernels change
 their tiles (75 to 148 tiles: small ones for flow, large ones for the species
 kernel of a periodic box; above 148 large ones throughout), with partial tiles
-in every direction: odd extents and even ones (rows staged by bulk copies), and
-inflow/outflow faces. Against the oracle.
+in every direction: odd extents and even ones (rows staged by bulk copies), rows
+that wrap several times within a tile, inflow/outflow faces and walls, with
+and without the transport switches. Against the oracle.
 
 Bound: 1e-10 of the field's maximum (right-hand side and two steps), as in the
 other parity tests."""
@@ -15,11 +16,19 @@ pytestmark = pytest.mark.gpu
 
 ALL = dict(mixw=True, mixp=True, soret=True, dufour=True)
 
-# (case, shape, switches on, steps)
+# (case, shape, switches on, steps); a box of 6 points in x resolves the
+# kernels with two points and leaves the physical range: right-hand side only
 CASES = [
     ("h2_pool", (65, 33, 17), False, 2),  # 135 tiles
     ("h2_pool", (66, 35, 19), False, 2),  # 150, bulk rows
     ("flame_inout", (45, 33, 25), True, 2),  # 130
+    ("h2_pool", (69, 61, 37), True, 2),  # 456
+    ("h2_pool", (70, 61, 37), False, 2),  # 456, bulk rows
+    ("h2_pool", (6, 42, 60), True, 0),  # 180, bulk rows that wrap
+    ("flame_inout", (69, 61, 37), False, 2),
+    ("flame_inout", (36, 61, 39), True, 2),  # 320, both ends' closures in one tile and across two
+    ("wall_box", (45, 68, 35), False, 2),  # 324
+    ("wall_box", (64, 41, 51), True, 2),  # 312
 ]
 
 
