@@ -120,6 +120,12 @@ int launch_thermo(const Geo& g, const Fields& f, const senga_chem* dchem, const 
   return 1;
 }
 
+cudaError_t load_thermo() {
+  return load_kernels(k_thermo<gen::Mech_onestep>, k_thermo<MechTables<2, true>>, k_thermo<MechTables<2, false>>,
+                      k_thermo_part<gen::Mech_h2, 1>, k_thermo_part<gen::Mech_h2, 2>,
+                      k_thermo_part<gen::Mech_h2_ref, 1>, k_thermo_part<gen::Mech_h2_ref, 2>);
+}
+
 void launch_batch_thermo(const BoxTable& boxes, const WorkItem* chunks, int nchunks, int grid, int mech,
                          const senga_chem* dchem, const senga_diff* ddiff, int nspec, int flmavt, cudaStream_t s) {
   if (mech == 1) {

@@ -253,6 +253,14 @@ bool make_map(CUtensorMap* m, const double* base, const Geo& g, int nk, unsigned
 
 }  // namespace
 
+cudaError_t load_stencils() {
+  return load_kernels(k_flow_line<true>, k_species_line<true>, k_species_rk_line<true>, k_flow_t<true, true>,
+                      k_flow_t<true, false>, k_flow_t<true, true, TileS>, k_flow_t<true, false, TileS>,
+                      k_species_t<true, 0>, k_species_t<true, 1>, k_species_t<true, 2>, k_species_t<true, 0, TileS>,
+                      k_species_rk_t<true, 0>, k_species_rk_t<true, 1>, k_species_rk_t<true, 2>,
+                      k_species_rk_t<true, 0, TileS>);
+}
+
 void launch_flow(const Geo& g, const Fields& f, int, cudaStream_t s, const ZDec& zd) {
   if (one_line(g, zd)) {
     if (g.per[0]) k_flow_line<true><<<line_tiles(g), Tile1::X, 0, s>>>(g, f);

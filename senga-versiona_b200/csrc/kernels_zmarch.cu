@@ -184,6 +184,8 @@ bool plane_map(CUtensorMap* m, const double* base, const Geo& g, int nk) {
 
 }  // namespace
 
+cudaError_t load_species_rk_z() { return load_kernels(k_species_rk_z); }
+
 // Launches the z-marching form when the box qualifies (all periodic, one
 // context, even nx, 16-byte aligned fields, the encoder available); returns
 // false otherwise so the caller launches the tiled form.

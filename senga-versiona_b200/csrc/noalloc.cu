@@ -23,8 +23,8 @@
 //     device addresses of the file-scope arrays (cudaGetSymbolAddress); make
 //     that first call before any stream capture. Under CUDA's lazy module
 //     loading (the default of recent CUDA releases) that first call is also
-//     when the array and the kernels' code are loaded onto the device, so a
-//     host that reserves all free device memory at start-up makes one call
+//     when the array and the code of the kernels of every box shape and
+//     mechanism are loaded onto the device, so a host that reserves all free device memory at start-up makes one call
 //     per device before it does (or runs with CUDA_MODULE_LOADING=EAGER);
 //   * the status word is required: it is the only place a TEMPER
 //     non-convergence is reported.
@@ -72,6 +72,15 @@ int setup(int dev, DevicePtrs& out) {
     if (e != cudaSuccess)
       return senga::fail(SENGA_ERR_CUDA, std::string("senga_rhs_noalloc: cudaGetSymbolAddress: ") +
                                              cudaGetErrorString(e));
+    // every form of every kernel, not only those of this call's box and
+    // mechanism: the host may reserve all device memory after this call
+    e = senga::load_thermo();
+    if (e == cudaSuccess) e = senga::load_thermo_tables();
+    if (e == cudaSuccess) e = senga::load_stencils();
+    if (e == cudaSuccess) e = senga::load_species_mma();
+    if (e == cudaSuccess) e = senga::load_species_rk_z();
+    if (e != cudaSuccess)
+      return senga::fail(SENGA_ERR_CUDA, std::string("senga_rhs_noalloc: loading kernels: ") + cudaGetErrorString(e));
     p.ready = true;
   }
   out = p;

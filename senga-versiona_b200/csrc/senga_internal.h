@@ -162,6 +162,21 @@ int launch_thermo(const Geo& g, const Fields& f, const senga_chem* dchem, const 
 // the table-driven form of any mechanism of more than two species
 int launch_thermo_tables(const Geo& g, const Fields& f, const senga_chem* dchem, const senga_diff* ddiff, int nspec,
                          int flmavt, cudaStream_t s);
+// Load the code of every kernel that a right-hand side of a periodic box can
+// launch, whatever its shape and mechanism, onto the current device (under
+// lazy module loading a kernel's code is otherwise loaded at its first launch).
+cudaError_t load_thermo();
+cudaError_t load_thermo_tables();
+cudaError_t load_stencils();
+cudaError_t load_species_mma();
+cudaError_t load_species_rk_z();
+template <class... K>
+cudaError_t load_kernels(K... kernels) {
+  cudaFuncAttributes a;
+  cudaError_t e = cudaSuccess;
+  ((e = e == cudaSuccess ? cudaFuncGetAttributes(&a, kernels) : e), ...);
+  return e;
+}
 void launch_flow(const Geo& g, const Fields& f, int nspec, cudaStream_t s, const ZDec& zd = ZDec{});
 void launch_species_a(const Geo& g, const Fields& f, int nspec, cudaStream_t s, const ZDec& zd = ZDec{});
 void launch_species_b_rk(const Geo& g, const Fields& f, int nspec, const RK& rk, cudaStream_t s,

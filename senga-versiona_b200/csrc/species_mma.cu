@@ -382,6 +382,8 @@ bool species_mma_ok(const Geo& g, const Fields& f, const ZDec& zd) {
          al16(f.uin);
 }
 
+cudaError_t load_species_mma() { return load_kernels(k_species_mma); }
+
 void launch_species_mma(const Geo& g, const Fields& f, int nspec, cudaStream_t s) {
   static bool attr[64] = {};
   int dev = 0;

@@ -225,6 +225,8 @@ __global__ void __launch_bounds__(kTabBlock) k_tab_chrate(Geo g, Fields f, const
 
 }  // namespace
 
+cudaError_t load_thermo_tables() { return load_kernels(k_tab_temper, k_tab_mixture, k_tab_chrate); }
+
 int launch_thermo_tables(const Geo& g, const Fields& f, const senga_chem* dchem, const senga_diff* ddiff, int nspec,
                          int flmavt, cudaStream_t s) {
   const unsigned grid = (unsigned)((g.n + kTabBlock - 1) / kTabBlock);

@@ -16,7 +16,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from conftest import rel_linf
+from conftest import ROOT, rel_linf
 
 pytestmark = pytest.mark.gpu
 
@@ -155,3 +155,64 @@ def test_rhs_noalloc_refuses_stream_capture():
     assert rc == 5
     assert b"captured" in senga.lib.senga_last_error()
     torch.cuda.synchronize(dev)
+
+
+def test_rhs_noalloc_first_call_loads_every_kernel():
+    """The first call loads the code of all kernels, so that a host may reserve
+    the remaining device memory after it: in a fresh process, later calls with
+    another mechanism or box shape (a 1D line, a box of few tiles, an odd one)
+    load none. The profiler reports each load of a kernel's code."""
+    import subprocess
+    import sys
+
+    run = subprocess.run([sys.executable, "-c", _FIRST_CALLS], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stderr[-2000:]
+    assert "later loads 0" in run.stdout, run.stdout
+
+
+_FIRST_CALLS = """
+import ctypes as C, os, sys
+sys.path.insert(0, os.path.join(os.getcwd(), "senga-versiona_b200"))
+import numpy as np, torch
+import cases, senga
+from torch.profiler import ProfilerActivity, profile
+
+dev = torch.device("cuda", 0)
+stream = torch.cuda.current_stream(dev).cuda_stream
+
+
+def args(name, shape):
+    c = dict(cases.make_case(name, n=16, seed=3))
+    nx, ny, nz = shape
+    chem = senga.Chem(c["chem"])
+    diff = senga.Diff(c["diff"], chem)
+    cfg = senga.make_config(shape, c["lengths"], c["dt"])
+    cut = (slice(None, nz), slice(None, ny), slice(None, nx))
+    state = torch.from_numpy(np.ascontiguousarray(c["fields"][(slice(None),) + cut])).to(dev)
+    t = torch.from_numpy(np.ascontiguousarray(c["T"][cut])).to(dev)
+    itn = torch.from_numpy(np.ascontiguousarray(c["itn"][cut])).to(dev)
+    return cfg, chem, diff, state, t, itn, torch.empty_like(state), torch.zeros(1, dtype=torch.int32, device=dev)
+
+
+def call(a):
+    cfg, chem, diff, state, t, itn, rhs, status = a
+    senga._check(senga.lib.senga_rhs_noalloc(C.byref(cfg), C.byref(chem.t), C.byref(diff.t), state.data_ptr(),
+                                             t.data_ptr(), itn.data_ptr(), rhs.data_ptr(), status.data_ptr(), stream),
+                 "senga_rhs_noalloc")
+    torch.cuda.synchronize(dev)
+
+
+def loads(a):
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
+        call(a)
+    return sum("Lazy Function Loading" in e.name for e in p.events())
+
+
+boxes = [args(n, s) for n, s in (("ignition32", (16, 16, 16)), ("ignition32", (16, 1, 1)), ("h2_kernels", (16, 16, 16)),
+                                 ("h2_kernels", (15, 14, 1)), ("h2_kernels", (16, 1, 1)))]
+torch.cuda.synchronize(dev)
+call(boxes[0])
+later = sum(loads(a) for a in boxes[1:])
+os.environ["SENGA_MECH"] = "generic"
+print("later loads", later + sum(loads(a) for a in boxes[:3]))
+"""
