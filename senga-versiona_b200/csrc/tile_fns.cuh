@@ -71,18 +71,12 @@ struct Tile1 {
   using Slab = Line<X>;
   using Col = PointColumn;
 };
-// Tile3 for boxes of fewer tiles than SMs: the same plane of points, half the
-// planes or rows, so that twice the CTAs share the work of a box that leaves
-// SMs idle (kernels_tiled.cu: small_tiles).
-#ifndef SENGA_SMALL_Y
-#define SENGA_SMALL_Y 8
-#endif
-#ifndef SENGA_SMALL_Z
-#define SENGA_SMALL_Z 1
-#endif
+// Tile3 for boxes of fewer tiles than SMs: one plane of the same points, so that
+// twice the CTAs share the work of a box that leaves SMs idle
+// (kernels_tiled.cu: small_tiles).
 struct TileS {
   static constexpr bool kLine = false;
-  static constexpr int X = FX, Y = SENGA_SMALL_Y, Z = SENGA_SMALL_Z;
+  static constexpr int X = FX, Y = FY, Z = 1;
   using Star = tile::Star<X, Y, Z>;
   using Box = tile::Box<X, Y, Z>;
   using XRow = tile::XRow<X, Y, Z>;

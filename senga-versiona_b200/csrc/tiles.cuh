@@ -6,8 +6,9 @@
 // points, the half-width of the 11-point stencils), then all derivatives of
 // that field at the tile's points are read from shared memory. Halo points of
 // periodic directions are wrapped into the domain (the single-rank halo copy
-// of src/parfer.f:840-873); in a bounded direction they are clamped and never
-// read, because the one-sided closures only look inward.
+// of src/parfer.f:840-873). In a bounded direction they are clamped: the
+// interior scheme reads them at the points next to an end, where its result is
+// replaced by that of a one-sided closure, which only looks inward.
 //
 // Buffer layouts (doubles; SX = TX + 2*XH, one column more than the 5-point
 // halo on each side so that every row starts on a 16-byte boundary):
@@ -41,7 +42,7 @@ struct Origin {
 };
 
 // Fold a coordinate into the domain: periodic wrap, or clamp (bounded
-// directions: the clamped halo values are never read by the closures).
+// directions: no result that is kept depends on the clamped halo values).
 __device__ __forceinline__ int fold(int c, int n, int per) {
   if (per) {
     while (c < 0) c += n;
@@ -589,6 +590,7 @@ struct Line {
   __device__ void stage(const Folds<TX, 1, 1>& fo, const F& f) const {
     stage_rows<TX + 2 * H, -H, 1, NW>(p + (XH - H), SX, fo, [](int, int& y, int& z, int& d) { y = z = d = 0; }, f);
   }
+  // one row: a single round of loads, whatever UB the tile kernels ask for
   template <int NW, int UB, class F>
   __device__ void stage3(const Line& b, const Line& c, const Folds<TX, 1, 1>& fo, const F& f) const {
     stage_rows3<TX + 2 * H, -H, 1, NW, 1>(p + (XH - H), b.p + (XH - H), c.p + (XH - H), SX, fo,
@@ -646,13 +648,13 @@ __device__ __forceinline__ TP make_tp(const Geo& g, const Origin& o, int x, int 
 // pass per row (six to eleven) for every x derivative of the end tiles; here
 // every lane evaluates the interior scheme and the end lanes one more pass
 // with their own weights and offsets. The terms and their order are those of
-// the switch, so the values are bit for bit the same. 128^3 H2 flame: flow
-// 1423 -> 814, species 1401 -> 934 us per launch.
+// the switch. 128^3 H2 flame: flow 1423 -> 814, species 1401 -> 934 us per
+// launch.
 struct EndTables {
   // [point 0..4 from the left end, 5..9 from the right][term]; the right
-  // end's one-sided first-derivative rows hold -weight and swapped offsets:
-  // -w (v(q) - v(p)) is w (v(p) - v(q)) bit for bit, and where v is a product
-  // the one that the switch's form contracted into the subtraction stays so
+  // end's one-sided first-derivative rows hold -weight and swapped offsets
+  // (the same number), so that where v is a product it is the same one of the
+  // two as in the switch that the compiler can contract into the subtraction
   double w1[10][5];
   double w2[5][5], wm[5][5];  // [distance from the end][term]
   // offsets + 5 in 4 bits: term j's first value at bit 4j, second at 20 + 4j;

@@ -102,27 +102,29 @@ __global__ void __launch_bounds__(TS::X* TS::Y) k_mixt_grad(Geo g, MixtParams m)
   fo.init(g, o);
   tile_sync();
   const int64_t n = g.n;
-  const double* const F[3] = {m.w ? m.lng[0] : nullptr, m.p ? m.lng[1] : nullptr, m.t ? m.lng[2] : nullptr};
+  auto of = [](int b, double* const (&a)[3]) { return b == 0 ? a[0] : b == 1 ? a[1] : a[2]; };
+  const bool on[3] = {m.w != 0, m.p != 0, m.t != 0};
 #pragma unroll
   for (int b = 0; b < 3; ++b)
-    if (F[b]) Slab{sm + b * Slab::SIZE}.template stage<TS::X * TS::Y / 32>(fo, Ld{F[b]});
+    if (on[b]) Slab{sm + b * Slab::SIZE}.template stage<TS::X * TS::Y / 32>(fo, Ld{m.lng[b]});
   tile_sync();
 #pragma unroll 1
   for (int b = 0; b < 3; ++b) {
-    if (!F[b]) continue;
+    if (!(b == 0 ? on[0] : b == 1 ? on[1] : on[2])) continue;
     const Slab s{sm + b * Slab::SIZE};
+    double *const g1 = of(b, m.g1), *const g2 = of(b, m.g2);
     typename TS::Col c;
-    c.load(fo, tx, ty, Ld{F[b]});
+    c.load(fo, tx, ty, Ld{of(b, m.lng)});
 #pragma unroll
     for (int z = 0; z < TS::Z; ++z) {
       const TP t = make_tp(g, o, tx, ty, z);
       if (!t.valid) continue;
       const bool dif = !P && (face_bits(g, t.gx) & BF_DIF);
-      m.g1[b][t.q] = d1<0, P>(g, t, s);
-      m.g1[b][n + t.q] = d1<1, P>(g, t, s);
-      m.g1[b][2 * n + t.q] = d1z<P>(g, t, c);
+      g1[t.q] = d1<0, P>(g, t, s);
+      g1[n + t.q] = d1<1, P>(g, t, s);
+      g1[2 * n + t.q] = d1z<P>(g, t, c);
       const double d2x = dif ? 0.0 : d2<0, P>(g, t, s);
-      m.g2[b][t.q] = d2x + d2<1, P>(g, t, s) + d2z<P>(g, t, c);
+      g2[t.q] = d2x + d2<1, P>(g, t, s) + d2z<P>(g, t, c);
     }
   }
 }
