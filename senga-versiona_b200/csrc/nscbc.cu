@@ -67,21 +67,34 @@ __device__ __forceinline__ double at(const Geo& g, const ZDec& zd, const double*
   }
   return a[base + (int64_t)i + (int64_t)g.nx * (j + (int64_t)g.ny * k)];
 }
-// Derivative of (a - c0) along DIR; c0 = 0 (exact) for every field but the
-// pressure, whose gradient RHSVEL takes of p - p(1,1,1) (src/rhsvel.f:730-752).
-// A function, not inlined: a face kernel of a few warps runs its code once and
-// waits for the instructions, and with some 30 inlined copies of the closures
-// that wait was the kernel (23 us for the two points of a 1D box, 15 us so).
+// Derivatives of (a - c0) along DIR; c0 is not zero for the pressure only, whose
+// gradient RHSVEL takes of p - p(1,1,1) (src/rhsvel.f:730-752). A face kernel of
+// a few warps runs its code once and waits for the instructions: with some 30
+// inlined copies of the closures that wait was the kernel (24 us for the two
+// points of a 1D box). The x derivatives, one row of the closures each, are
+// inlined; the y and z ones, folded neighbours and all, are functions, skipped
+// where there is one point: 1D 24.4 -> 11.7 us, 64x64x18 31.6 -> 27.9,
+// 32x160x160 77 -> 68 (all of them functions: 15.2, 31.8 and 73.8).
 template <int DIR>
-__device__ __noinline__ double dd_sub(const Geo& g, const ZDec& zd, const double* a, double c0, int i, int j, int k) {
-  const int c = DIR == 0 ? i : DIR == 1 ? j : k;
-  const int n = DIR == 0 ? g.nx : DIR == 1 ? g.ny : g.nz;
-  if (DIR == 1 ? n == 1 : DIR == 2 && n == 1 && zd.nr <= 1) return 0.0;  // differences of a point with itself
-  return d1core([&](int m) { return at<DIR>(g, zd, a, i, j, k, m) - c0; }, c, n, DIR == 0 ? g.per[0] : 1) * g.ovd[DIR];
+__device__ __noinline__ double dd_core(const Geo& g, const ZDec& zd, const double* a, double c0, int i, int j, int k) {
+  const int c = DIR == 1 ? j : k, n = DIR == 1 ? g.ny : g.nz;
+  if (n == 1 && (DIR == 1 || zd.nr <= 1)) return 0.0;  // differences of a point with itself
+  return d1core([&](int m) { return at<DIR>(g, zd, a, i, j, k, m) - c0; }, c, n, 1);
+}
+template <int DIR>
+__device__ __forceinline__ double dd_sub(const Geo& g, const ZDec& zd, const double* a, double c0, int i, int j,
+                                         int k) {
+  if constexpr (DIR == 0)
+    return d1core([&](int m) { return at<DIR>(g, zd, a, i, j, k, m) - c0; }, i, g.nx, g.per[0]) * g.ovd[0];
+  else
+    return dd_core<DIR>(g, zd, a, c0, i, j, k) * g.ovd[DIR];
 }
 template <int DIR>
 __device__ __forceinline__ double dd(const Geo& g, const ZDec& zd, const double* a, int i, int j, int k) {
-  return dd_sub<DIR>(g, zd, a, 0.0, i, j, k);
+  if constexpr (DIR == 0)
+    return d1core([&](int m) { return at<DIR>(g, zd, a, i, j, k, m); }, i, g.nx, g.per[0]) * g.ovd[0];
+  else
+    return dd_core<DIR>(g, zd, a, 0.0, i, j, k) * g.ovd[DIR];
 }
 
 // h_k(T) per unit mass of interval `it` (AMASCH polynomial, boundt.f:316-324)
