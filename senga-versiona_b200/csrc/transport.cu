@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(kMixBlock) k_mixt_pre(Geo g, Fields f, MixtPar
 // Gradients of the logarithms on the species kernels' tiles: each field staged
 // once with its x and y halos, the z column in registers (one thread a point
 // over global memory re-folded every neighbour and switched over the closure
-// rows: 64 us on 64x56x48, 15 us so; 1001-point line 58 -> 4.4 us).
+// rows: 64 us on 64x56x48, 11 us so; 96x80x64 24 us; 1001-point line 58 -> 4.4 us).
 constexpr int MX = 32, MY = 8, MZ = 2;
 struct MTile3 {
   static constexpr bool kLine = false;
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(TS::X* TS::Y) k_mixt_grad(Geo g, MixtParams m)
       const TP t = make_tp(g, o, tx, ty, z);
       if (!t.valid) continue;
       const bool dif = !P && (face_bits(g, t.gx) & BF_DIF);
-      g1[t.q] = d1<0, P>(g, t, s);
+      g1[t.q] = d1<0, P, kGrad>(g, t, s);
       g1[n + t.q] = d1<1, P>(g, t, s);
       g1[2 * n + t.q] = d1z<P>(g, t, c);
       const double d2x = dif ? 0.0 : d2<0, P>(g, t, s);
@@ -272,7 +272,8 @@ __global__ void __launch_bounds__(TS::X* TS::Y, TS::kLine ? 1 : 2) k_mixt_specie
       const double f2 = lG[z] * s7;
       vt[z] = vt[z] + f1 + f2;
       ea[z] = ea[z] + f1 * u + (dH[0] * gG[z][0] + dH[1] * gG[z][1] + dH[2] * gG[z][2]) * s7 + f2 * u;
-      if (t.valid) f.wdot[k * n + t.q] += f1 + f2;
+      // (on lines the sum that the compiler forms on the tiles, written out)
+      if (t.valid) f.wdot[k * n + t.q] += TS::kLine ? fma(lG[z], s7, f1) : f1 + f2;
     }
   }
 #pragma unroll
