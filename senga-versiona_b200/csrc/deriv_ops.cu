@@ -4,9 +4,9 @@
 // false; periodic neighbours folded into the domain) or on halo-extended
 // ones (BIG = true; five points per side, read as the caller filled them).
 //
-// What bounds them: 16 bytes a point of compulsory traffic (9 us for a
-// 192 x 160 x 120 field at 6.5 TB/s, less while the operand sits in L2). The
-// neighbours come through L1, two 128-byte wavefronts per warp and load, so
+// What bounds them: the latency of the neighbours' loads (6 to 10 warps wait for
+// one per issue, at half the warp slots; L1 31 to 62% busy, DRAM 8 to 12%). The
+// floor is 16 bytes a point, 9 us for a 192 x 160 x 120 field at 6.5 TB/s. So
 // what has to go is everything else: one thread marches over the z planes of
 // its (x, y), with the in-plane neighbour offsets folded once into registers,
 // and the z operators slide a register window so that every value is loaded
