@@ -262,13 +262,6 @@ def poly_expr(coefs, var):
     return e
 
 
-def poly_pinned(coefs, var, fused):
-    """As poly_expr, with the last step written out: one fused operation, or a
-    product and a sum."""
-    e = poly_expr(coefs[1:], var)
-    return f"fma({e}, {var}, {h(coefs[0])})" if fused else f"__dadd_rn(__dmul_rn({e}, {var}), {h(coefs[0])})"
-
-
 def sel(it_var, a, b):
     """The value of interval it_var: a select, or the literal itself inside a
     function whose template mode IM fixes the interval (see `modes`)."""
@@ -757,12 +750,6 @@ def gen(tag, c, d, shared=True):
     return "\n".join(o)
 
 
-# Species pairs of the H2 mechanism (O2-H, O-H, OH-H, O-N2, OH-N2) whose shared
-# polynomial ends in a fused operation; those of the other pairs end in a
-# rounded product.
-FUSED = ((1, 5), (3, 5), (4, 5), (3, 8), (4, 8))
-
-
 def gen_ref(tag, c, d):
     """The shared policy's transport and rates with nothing shared: one exp per
     polynomial and per rate, one divide per quotient. Contexts with the adaptive
@@ -805,17 +792,9 @@ def gen_ref(tag, c, d):
         w(f"    sumy += y[{s}] + {h(DFCTOL)};")
     for s in range(ns):
         w(f"    double den{s} = 0.0;")
-    # Pairs whose polynomials differ in the constant only share all the steps
-    # but the last, and the compiler may round the shared product once or fuse
-    # it into each sum. What it had chosen is written out, digit for digit, so
-    # that no later build moves the step size (see FUSED).
-    pairs = [((s, t), d["diffco"][s][t]) for s in range(ns) for t in range(s + 1, ns)]
-    shared = {m for _, mem in groups_of(pairs) if len(mem) > 1 for m in mem}
     for s in range(ns):
         for t in range(s + 1, ns):
-            co = d["diffco"][s][t]
-            pe = poly_pinned(co, "lt", (s, t) in FUSED) if (s, t) in shared else poly_expr(co, "lt")
-            w(f"    {{ const double inv = exp(-{pe}) * povr;")
+            w(f"    {{ const double inv = exp(-{poly_expr(d['diffco'][s][t], 'lt')}) * povr;")
             w(f"      den{s} += (y[{t}] + {h(DFCTOL)}) * {h(c['ovwmol'][t])} * inv;")
             w(f"      den{t} += (y[{s}] + {h(DFCTOL)}) * {h(c['ovwmol'][s])} * inv; }}")
     for s in range(ns):

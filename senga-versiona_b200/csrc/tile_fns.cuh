@@ -197,7 +197,7 @@ __device__ __forceinline__ void flow_tile(const Geo& g, const Fields& f, const O
       divm[z] = dv;
       const double s4 = bE.v(t.x, t.y, t.z) * dv + d1p<0, P>(g, t, bE, bru) + d1p<1, P>(g, t, bE, brv) +
                         d1p<2, P>(g, t, bE, brw);
-      rE[z] = -0.5 * (s4 + d1<0, P, kGrad>(g, t, bE) * bru.v(t.x, t.y, t.z) + d1<1, P>(g, t, bE) * brv.v(t.x, t.y, t.z) +
+      rE[z] = -0.5 * (s4 + d1<0, P>(g, t, bE) * bru.v(t.x, t.y, t.z) + d1<1, P>(g, t, bE) * brv.v(t.x, t.y, t.z) +
                       d1<2, P>(g, t, bE) * brw.v(t.x, t.y, t.z));
     }
     tile_sync();
@@ -238,7 +238,7 @@ __device__ __forceinline__ void flow_tile(const Geo& g, const Fields& f, const O
 #pragma unroll
       for (int z = 0; z < FZ; ++z) {
         const TP& t = tp[z];
-        const double px = d1<0, P, kGrad>(g, t, bP), py = d1<1, P>(g, t, bP), pz = d1<2, P>(g, t, bP);
+        const double px = d1<0, P>(g, t, bP), py = d1<1, P>(g, t, bP), pz = d1<2, P>(g, t, bP);
         rU[z] = -px;
         rV[z] = -py;
         rW[z] = -pz;
@@ -649,7 +649,7 @@ __device__ __forceinline__ void species_tile(const Geo& g, const Fields& f, int 
         const int e = P ? -1 : end_row(g, t.gx);
         if (!P && e >= 0) {
           auto y = [&](int m) { return bS.v(t.x + m, t.y, t.z); };
-          d1px = d1end<TS::kLine ? kProd : kPlain>([&](int m) { return bS.v(t.x + m, t.y, t.z) * bru.v(t.x + m, t.y, t.z); }, e);
+          d1px = d1end([&](int m) { return bS.v(t.x + m, t.y, t.z) * bru.v(t.x + m, t.y, t.z); }, e);
           dyx = d1end(y, e);
           d2x = d2end(y, e);
         }

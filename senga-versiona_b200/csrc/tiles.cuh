@@ -650,28 +650,16 @@ __device__ __forceinline__ TP make_tp(const Geo& g, const Origin& o, int x, int 
 // with their own weights and offsets. The terms and their order are those of
 // the switch. 128^3 H2 flame: flow 1423 -> 814, species 1401 -> 934 us per
 // launch.
-// The first two terms of a row are summed as fma(first, second product), so
-// their order decides a rounding. The orders here are those that the switch
-// had at each place (the compiler had chosen them differently), bit for bit:
-// the adaptive time step's error norm cancels all but the last digits, and
-// with one order throughout it moved the step size of a 1001-point flame by
-// up to 2e-10 in ten steps. First derivatives come in three sets: kPlain
-// (second term of the row of the third point first), kGrad (no row swapped:
-// the gradients of pressure, energy and the transport switches' logarithms)
-// and, on lines, kProd (second term of the row of the second point first:
-// fluxes formed as products; a second set in the species kernel of wider boxes
-// costs it 4%).
-enum { kPlain = 0, kGrad = 1, kProd = 2 };
 struct EndTables {
-  // [set][point 0..4 from the left end, 5..9 from the right][term]; the right
+  // [point 0..4 from the left end, 5..9 from the right][term]; the right
   // end's one-sided first-derivative rows hold -weight and swapped offsets
   // (the same number), so that where v is a product it is the same one of the
   // two as in the switch that the compiler can contract into the subtraction
-  double w1[3][10][5];
+  double w1[10][5];
   double w2[5][5], wm[5][5];  // [distance from the end][term]
   // offsets + 5 in 4 bits: term j's first value at bit 4j, second at 20 + 4j;
   // as w1 and by point
-  uint64_t o1[3][10], o2[10];
+  uint64_t o1[10], o2[10];
 };
 constexpr uint64_t end_offs(int p0, int p1, int p2, int p3, int p4, int q0, int q1, int q2, int q3, int q4) {
   const int v[10] = {p0, p1, p2, p3, p4, q0, q1, q2, q3, q4};
@@ -680,38 +668,33 @@ constexpr uint64_t end_offs(int p0, int p1, int p2, int p3, int p4, int q0, int 
   return r;
 }
 constexpr uint64_t kCen2 = end_offs(1, 2, 1, 1, 1, -1, -2, -1, -1, -1);
-constexpr uint64_t kCen2s = end_offs(2, 1, 2, 2, 2, -2, -1, -2, -2, -2);  // terms swapped
 constexpr uint64_t kCen3 = end_offs(1, 2, 3, 1, 1, -1, -2, -3, -1, -1);
 constexpr uint64_t kCen4 = end_offs(1, 2, 3, 4, 1, -1, -2, -3, -4, -1);
-constexpr uint64_t kOne0 = end_offs(1, 2, 3, 4, 1, 0, 0, 0, 0, 0), kOne0r = end_offs(-1, -2, -3, -4, -1, 0, 0, 0, 0, 0);
-constexpr uint64_t kOne1 = end_offs(-1, 1, 2, 3, -1, 0, 0, 0, 0, 0), kOne1r = end_offs(1, -1, -2, -3, 1, 0, 0, 0, 0, 0);
-constexpr uint64_t kOne1s = end_offs(1, -1, 2, 3, 1, 0, 0, 0, 0, 0), kOne1rs = end_offs(-1, 1, -2, -3, -1, 0, 0, 0, 0, 0);
-// rows of one end: the sign of the one-sided ones, and which rows are swapped
-#define SENGA_END_ROWS(S, P2A, P2B, P3A, P3B)                       \
-  {S fdc::p1a, S fdc::p1b, S fdc::p1c, S fdc::p1d, 0.0},            \
-      {S fdc::P2A, S fdc::P2B, S fdc::p2c, S fdc::p2d, 0.0},        \
-      {fdc::P3A, fdc::P3B, 0.0, 0.0, 0.0},                          \
-      {fdc::p4a, fdc::p4b, fdc::p4c, 0.0, 0.0}, {fdc::p5a, fdc::p5b, fdc::p5c, fdc::p5d, 0.0}
 static __device__ const EndTables kEnd = {
-    {{SENGA_END_ROWS(+, p2a, p2b, p3b, p3a), SENGA_END_ROWS(-, p2a, p2b, p3b, p3a)},
-     {SENGA_END_ROWS(+, p2a, p2b, p3a, p3b), SENGA_END_ROWS(-, p2a, p2b, p3a, p3b)},
-     {SENGA_END_ROWS(+, p2b, p2a, p3a, p3b), SENGA_END_ROWS(-, p2b, p2a, p3a, p3b)}},
-    {{fdc::s1b, fdc::s1a, fdc::s1c, fdc::s1d, fdc::s1e},
+    {{fdc::p1a, fdc::p1b, fdc::p1c, fdc::p1d, 0.0},
+     {fdc::p2a, fdc::p2b, fdc::p2c, fdc::p2d, 0.0},
+     {fdc::p3a, fdc::p3b, 0.0, 0.0, 0.0},
+     {fdc::p4a, fdc::p4b, fdc::p4c, 0.0, 0.0},
+     {fdc::p5a, fdc::p5b, fdc::p5c, fdc::p5d, 0.0},
+     {-fdc::p1a, -fdc::p1b, -fdc::p1c, -fdc::p1d, 0.0},
+     {-fdc::p2a, -fdc::p2b, -fdc::p2c, -fdc::p2d, 0.0},
+     {fdc::p3a, fdc::p3b, 0.0, 0.0, 0.0},
+     {fdc::p4a, fdc::p4b, fdc::p4c, 0.0, 0.0},
+     {fdc::p5a, fdc::p5b, fdc::p5c, fdc::p5d, 0.0}},
+    {{fdc::s1a, fdc::s1b, fdc::s1c, fdc::s1d, fdc::s1e},
      {fdc::s2a, fdc::s2b, fdc::s2c, fdc::s2d, fdc::s2e},
      {fdc::s3a, fdc::s3b, 0.0, 0.0, 0.0},
      {fdc::s4a, fdc::s4b, fdc::s4c, 0.0, 0.0},
      {fdc::s5a, fdc::s5b, fdc::s5c, fdc::s5d, 0.0}},
     {{0.0, 0.0, 0.0, 0.0, 0.0},
      {0.0, 0.0, 0.0, 0.0, 0.0},
-     {fdc::m3b, fdc::m3a, 0.0, 0.0, 0.0},
+     {fdc::m3a, fdc::m3b, 0.0, 0.0, 0.0},
      {fdc::m4a, fdc::m4b, fdc::m4c, 0.0, 0.0},
      {fdc::m5a, fdc::m5b, fdc::m5c, fdc::m5d, 0.0}},
-    {{kOne0, kOne1, kCen2s, kCen3, kCen4, kOne0r, kOne1r, kCen2s, kCen3, kCen4},
-     {kOne0, kOne1, kCen2, kCen3, kCen4, kOne0r, kOne1r, kCen2, kCen3, kCen4},
-     {kOne0, kOne1s, kCen2, kCen3, kCen4, kOne0r, kOne1rs, kCen2, kCen3, kCen4}},
-    {end_offs(2, 1, 3, 4, 5, 0, 0, 0, 0, 0), end_offs(-1, 1, 2, 3, 4, 0, 0, 0, 0, 0), kCen2, kCen3, kCen4,
-     end_offs(-2, -1, -3, -4, -5, 0, 0, 0, 0, 0), end_offs(1, -1, -2, -3, -4, 0, 0, 0, 0, 0), kCen2, kCen3, kCen4}};
-#undef SENGA_END_ROWS
+    {end_offs(1, 2, 3, 4, 1, 0, 0, 0, 0, 0), end_offs(-1, 1, 2, 3, -1, 0, 0, 0, 0, 0), kCen2, kCen3, kCen4,
+     end_offs(-1, -2, -3, -4, -1, 0, 0, 0, 0, 0), end_offs(1, -1, -2, -3, 1, 0, 0, 0, 0, 0), kCen2, kCen3, kCen4},
+    {end_offs(1, 2, 3, 4, 5, 0, 0, 0, 0, 0), end_offs(-1, 1, 2, 3, 4, 0, 0, 0, 0, 0), kCen2, kCen3, kCen4,
+     end_offs(-1, -2, -3, -4, -5, 0, 0, 0, 0, 0), end_offs(1, -1, -2, -3, -4, 0, 0, 0, 0, 0), kCen2, kCen3, kCen4}};
 // row of the tables for the point at gx, -1: interior scheme. Points past the
 // end of a partial tile (never stored) evaluate as the last point, so a closure
 // never reaches outside the staged halo.
@@ -721,10 +704,10 @@ __device__ __forceinline__ int end_row(const Geo& g, int gx) {
 }
 __device__ __forceinline__ int end_p(uint64_t o, int j) { return (int)(o >> (4 * j) & 15u) - 5; }
 __device__ __forceinline__ int end_q(uint64_t o, int j) { return (int)(o >> (20 + 4 * j) & 15u) - 5; }
-template <int SET = kPlain, class V>
+template <class V>
 __device__ __forceinline__ double d1end(const V& v, int e) {
-  const double* const w = kEnd.w1[SET][e];
-  const uint64_t o = __ldg(&kEnd.o1[SET][e]);
+  const double* const w = kEnd.w1[e];
+  const uint64_t o = __ldg(&kEnd.o1[e]);
   auto d = [&](int j) { return v(end_p(o, j)) - v(end_q(o, j)); };
   return __ldg(w) * d(0) + __ldg(w + 1) * d(1) + __ldg(w + 2) * d(2) + __ldg(w + 3) * d(3) + __ldg(w + 4) * d(4);
 }
@@ -741,7 +724,7 @@ template <class V2>
 __device__ __forceinline__ double dmend(const V2& v, int e) {
   using namespace fdc;
   const int c = e < 5 ? e : e - 5;
-  const uint64_t o = __ldg(&kEnd.o1[kPlain][e]);
+  const uint64_t o = __ldg(&kEnd.o1[e]);
   if (c >= 2) {
     const double* const w = kEnd.wm[c];
     auto dg = [&](int j) {
@@ -750,7 +733,7 @@ __device__ __forceinline__ double dmend(const V2& v, int e) {
     };
     return __ldg(w) * dg(0) + __ldg(w + 1) * dg(1) + __ldg(w + 2) * dg(2) + __ldg(w + 3) * dg(3);
   }
-  const double* const w = kEnd.w1[kPlain][c];
+  const double* const w = kEnd.w1[c];
   auto g2 = [&](int j) {
     const int a = e < 5 ? end_p(o, j) : 0, b = e < 5 ? 0 : end_p(o, j);
     return my1 * (v(a, 1) - v(a, -1) - v(b, 1) + v(b, -1)) + my2 * (v(a, 2) - v(a, -2) - v(b, 2) + v(b, -2));
@@ -762,12 +745,12 @@ __device__ __forceinline__ double dmend(const V2& v, int e) {
 // P = true: every direction is periodic (known at compile time, no closure
 // branch); P = false: x may be bounded (boxes bounded in y or z are refused
 // before any right-hand-side launch, so those directions are periodic).
-template <bool P, int SET = kPlain, class V>
+template <bool P, class V>
 __device__ __forceinline__ double d1x(const Geo& g, const TP& t, const V& v) {
   double r = d1core(v, 0, 0, 1);
   if constexpr (!P) {
     const int e = end_row(g, t.gx);
-    if (e >= 0) r = d1end<SET>(v, e);
+    if (e >= 0) r = d1end(v, e);
   }
   return r;
 }
@@ -780,10 +763,10 @@ __device__ __forceinline__ double d2x(const Geo& g, const TP& t, const V& v) {
   }
   return r;
 }
-template <int DIR, bool P, int SET = kPlain, class B>
+template <int DIR, bool P, class B>
 __device__ __forceinline__ double d1(const Geo& g, const TP& t, const B& b) {
   if constexpr (is_line<B> && DIR != 0) return 0.0;
-  if (DIR == 0) return d1x<P, SET>(g, t, [&](int m) { return b.v(t.x + m, t.y, t.z); }) * g.ovd[0];
+  if (DIR == 0) return d1x<P>(g, t, [&](int m) { return b.v(t.x + m, t.y, t.z); }) * g.ovd[0];
   if (DIR == 1) return d1core([&](int m) { return b.v(t.x, t.y + m, t.z); }, t.gy, g.ny, 1) * g.ovd[1];
   return d1core([&](int m) { return b.v(t.x, t.y, t.z + m); }, t.gz, g.nz, 1) * g.ovd[2];
 }
@@ -792,7 +775,7 @@ template <int DIR, bool P, class A, class B>
 __device__ __forceinline__ double d1p(const Geo& g, const TP& t, const A& a, const B& b) {
   if constexpr (is_line<B> && DIR != 0) return 0.0;
   if (DIR == 0)
-    return d1x<P, is_line<B> ? kProd : kPlain>(g, t, [&](int m) { return a.v(t.x + m, t.y, t.z) * b.v(t.x + m, t.y, t.z); }) * g.ovd[0];
+    return d1x<P>(g, t, [&](int m) { return a.v(t.x + m, t.y, t.z) * b.v(t.x + m, t.y, t.z); }) * g.ovd[0];
   if (DIR == 1)
     return d1core([&](int m) { return a.v(t.x, t.y + m, t.z) * b.v(t.x, t.y + m, t.z); }, t.gy, g.ny, 1) * g.ovd[1];
   return d1core([&](int m) { return a.v(t.x, t.y, t.z + m) * b.v(t.x, t.y, t.z + m); }, t.gz, g.nz, 1) * g.ovd[2];

@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(TS::X* TS::Y) k_mixt_grad(Geo g, MixtParams m)
       const TP t = make_tp(g, o, tx, ty, z);
       if (!t.valid) continue;
       const bool dif = !P && (face_bits(g, t.gx) & BF_DIF);
-      g1[t.q] = d1<0, P, kGrad>(g, t, s);
+      g1[t.q] = d1<0, P>(g, t, s);
       g1[n + t.q] = d1<1, P>(g, t, s);
       g1[2 * n + t.q] = d1z<P>(g, t, c);
       const double d2x = dif ? 0.0 : d2<0, P>(g, t, s);
@@ -272,8 +272,7 @@ __global__ void __launch_bounds__(TS::X* TS::Y, TS::kLine ? 1 : 2) k_mixt_specie
       const double f2 = lG[z] * s7;
       vt[z] = vt[z] + f1 + f2;
       ea[z] = ea[z] + f1 * u + (dH[0] * gG[z][0] + dH[1] * gG[z][1] + dH[2] * gG[z][2]) * s7 + f2 * u;
-      // (on lines the sum that the compiler forms on the tiles, written out)
-      if (t.valid) f.wdot[k * n + t.q] += TS::kLine ? fma(lG[z], s7, f1) : f1 + f2;
+      if (t.valid) f.wdot[k * n + t.q] += f1 + f2;
     }
   }
 #pragma unroll

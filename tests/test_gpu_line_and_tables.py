@@ -73,33 +73,3 @@ def test_table_driven_thermochemistry_matches_oracle(mavt, monkeypatch):
     if not mavt:
         c["diff"] = None
     _check(*_pair(c, False))
-
-
-# Step sizes after ten adaptive steps of a 1001-point flame with every transport
-# switch, by seed, as a build that evaluated the closures by a switch over the
-# rows, with its own inlined derivatives in every kernel, gave them.
-STEP_SIZES = {15: "0x1.ccb90281b5e29p-28", 17: "0x1.fab0017a87f81p-28", 23: "0x1.78b1086226543p-28",
-              24: "0x1.ff892892e47ffp-28"}
-
-
-@pytest.mark.parametrize("seed", sorted(STEP_SIZES))
-def test_adaptive_line_keeps_its_step_size(seed):
-    """The error norm cancels all but the last digits of the state, so another
-    order of two terms in a closure, or another fused operation in the
-    transport polynomials, moved the step size of these flames by 1e-12 to
-    2e-11 (2e-10 for other initial states). The orders are those of the build
-    that the values come from: 1e-13, a few hundred eps, is allowed."""
-    import cases
-    import senga
-
-    c = dict(cases.make_case("flame_inout", seed=seed, shape=(1001, 6, 6)))
-    cut = lambda a: np.ascontiguousarray(a[..., :1, :1, :])  # noqa: E731
-    chem = senga.Chem(c["chem"])
-    box = senga.Box((1001, 1, 1), c["lengths"], chem, senga.Diff(c["diff"], chem), c["dt"], nend=c["nend"],
-                    adaptive=True)
-    box.set_nscbc(c["bc"])
-    box.set_transport(**ALL)
-    box.upload(cut(c["fields"]), cut(c["T"]), cut(c["itn"]))
-    box.step(10)
-    got, want = float(box.tstep()[0]), float.fromhex(STEP_SIZES[seed])
-    assert abs(got - want) <= 1e-13 * want, abs(got - want) / want
